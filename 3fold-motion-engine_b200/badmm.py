@@ -2,11 +2,11 @@
 (src/motion_engine/ncp/ncp_batch_gpu.py:918-1313) behind its own method names.
 
 B independent contact problems of nc point contacts on nv generalised velocities (a legged
-stance: J (B, 3 nc, nv), M^-1 (B, nv, nv), v_free (B, nv), mu (B, nc)) are solved matrix-free
-with int64-accumulated M^-1 J^T products, by ADMM with a preconditioned CG x-step and a
-per-problem convergence mask, then differentiated by grad_affine.  ``b2c_admm_solve`` runs the
-whole of it -- set-up, iterations, refreshes, active set, both gradient directions -- with one
-warp per problem in ONE launch (the reference: 133 launches per ADMM iteration).
+stance: J (B, 3 nc, nv), M^-1 (B, nv, nv), v_free (B, nv), mu (B, nc)) are solved by ADMM with
+a preconditioned CG x-step and a per-problem convergence mask, then differentiated by
+grad_affine.  ``b2c_admm_solve`` runs the whole of it -- set-up, iterations, refreshes, active
+set, both gradient directions -- with one lane per contact in ONE launch (the reference: 133
+launches per ADMM iteration).
 
     s = BatchProxADMM(B, nv, nc).upload(J, Minv, v_free, mu, dt)
     s.set_rho("regime")

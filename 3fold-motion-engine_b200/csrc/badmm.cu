@@ -2,28 +2,41 @@
 // BatchProxADMMGPU (src/motion_engine/ncp/ncp_batch_gpu.py:918-1313, "NB").
 //
 // The reference runs every step as a separate kernel over the whole batch (133 launches per
-// ADMM iteration, ~35 000 graph nodes per step and gradient).  Here ONE warp owns one problem
-// for the whole solve: its J (3 nc x nv), M^-1 (nv x nv), M^-1 J^T, the dense Delassus G and
-// every vector live in the warp's shared memory, the set-up, the ADMM iterations, the refreshes,
-// the active set and both gradient directions run in one launch, and the only synchronisation
-// is __syncwarp.  The arithmetic is the reference's, float64:
-//  * set-up (NB:974-1000): b = J v_free, the scale bound kappa, M^-1 J^T (k_mj), G (k_gdense),
-//    G's spectrum by cyclic Jacobi in the fixed pair order (k_jacobi; the rotations' row and
-//    column updates spread over the lanes), the diagonal blocks and their largest eigenvalue
-//    (k_gd3, f_eigmax), eta and the per-contact step (k_eta), the bilateral regime test by a
-//    Cholesky solve (k_bilat), rho (k_rho), the block-Jacobi preconditioner (k_pjac);
-//  * the matrix-free product G x + (eta + rho) x (NB:326-388): y = J^T x per contact, then
-//    M^-1 y per contact rounded at a power-of-two scale 2^floor(log2(2^52 / (kappa |x|inf)))
-//    and summed in int64 (exact: the sum does not depend on the order), w = acc / scale, then J w;
+// ADMM iteration, ~35 000 graph nodes per step and gradient).  Here one launch runs everything
+// and ONE LANE OWNS ONE CONTACT: a problem of nc contacts takes 1, 2, 4 or 8 lanes (the power of
+// two that holds nc), a warp 32 / that many problems.  The arithmetic is float64:
+//  * set-up (NB:974-1000): b = J v_free, M^-1 J^T (k_mj) and the Delassus matrix G = J M^-1 J^T
+//    (k_gdense), the warp's problems one after the other; G's spectrum by cyclic Jacobi in the
+//    reference's row-cyclic order (k_jacobi; see spectrum()), the diagonal blocks and their
+//    largest eigenvalue (k_gd3, f_eigmax), eta and the per-contact step (k_eta), the bilateral
+//    regime test by a Cholesky solve (k_bilat), rho (k_rho), the block-Jacobi preconditioner
+//    (k_pjac);
+//  * the product G x + (eta + rho) x (NB:326-388) from G's rows, which a lane keeps in registers
+//    (3 rows of 3 nc): the lanes of a problem pass x through shared memory, everything else of a
+//    contact (its 3x3 preconditioner, cone projection, multiplier) is the lane's own, and a dot
+//    product is a 3-term sum and a butterfly over the problem's lanes;
 //  * ADMM (NB:466-543, 1075-1099): x-step by block-Jacobi preconditioned CG warm-started from
 //    the last x, z = proj_K(x + gamma / rho), gamma += rho (x - z), and every `refresh_every`
 //    iterations u = G z + b, the slip speeds, the natural residual and the convergence mask (a
 //    converged problem freezes x, z and gamma);
 //  * the gradient (NB:556-808, 1145-1206): the active set (open / stick / slip with its
 //    projector Z and diagonal D), the Schur preconditioner, and grad_affine -- the de Saxce
-//    sigma map is affine, so it is solved by 1 + n_calls - 2 + 1 applications of the
-//    CG-solved fixed-branch system and one (I - B) sigma = a elimination -- for the direction
-//    db = dt J M^-1 e_j (and v+'s response) and for mu at each problem's first slip contact.
+//    sigma map is affine, sigma -> a + B sigma: a from the direction with sigma = 0, B's columns
+//    from unit sigmas, one (I - B) sigma = a elimination and the response at that sigma, each a
+//    CG solve of the fixed-branch system -- for the direction db = dt J M^-1 e_j (and v+'s
+//    response) and for mu at each problem's first slip contact.  B does not depend on the
+//    direction, so both directions share its columns, and the solves run two at a time.
+//
+// What bounds it: the CG recurrence's dependent chain (exchange, 3 nc-term row sums, two dot
+// products, one division).  The time per CG step hardly depends on how many problems share a
+// warp, so the split puts as many there as there are contacts to own lanes, and leaves the
+// problem's matrix on chip.
+//
+// Measured on a B200 (200 iterations of 8 CG steps and both gradients; before: a warp per problem,
+// the products matrix-free), B problems of 4 contacts and 18 coordinates: B = 64 5.8 -> 1.24 ms,
+// B = 4096 20.8 -> 1.31 ms (forward alone 11.7 -> 1.00), B = 16384 112 -> 3.1 ms; at B = 4096, 1
+// contact 10.2 -> 0.91 ms, 8 contacts 81.9 -> 5.3 ms.  Error against 64-bit arithmetic on the
+// batch of 4096: 1.2e-14 of the worst output's norm (before: 3.3e-13).
 #include <math_constants.h>
 
 #include "b2c_common.cuh"
@@ -32,87 +45,46 @@ namespace b2c {
 namespace badmm {
 
 constexpr double kTiny = 1.0e-300;
-constexpr double kScaleBound = 4.503599627370496e15;  // 2^52
+constexpr unsigned kAll = 0xffffffffu;
 
-// one problem's working set in the warp's shared memory
-struct Env {
-    double *J, *Mi, *MJ, *G, *A, *yt, *wv, *vf;
-    double *bb, *x, *zv, *gam, *r, *zz, *pv, *Ap, *rhs, *tmp, *tmp2, *u, *pinh, *dbv, *ZtHp, *yv, *dlam, *Dv, *what,
-        *bw, *ev;
-    double *mu, *s, *eta, *rhoc, *slipf, *sig, *sigo, *siga, *res, *gnorm;
-    double *Gd, *Pj, *Zm, *Ps;  // 9 per contact, row-major
-    double *Bm, *Aw, *rw;
-    int *sidx;
-    int C, NV, M;
-    double kap, rho;
-    int mask, nslip;
+// the shapes of an instantiation: C contacts a problem
+template <int C>
+struct Dim {
+    static constexpr int M = 3 * C;                               // rows
+    static constexpr int L = C <= 1 ? 1 : C <= 2 ? 2 : C <= 4 ? 4 : 8;  // lanes of a problem
+    static constexpr int PW = 32 / L;                             // problems of a warp
+    static constexpr int XS = 2 * (((M + 1) / 2) | 1);            // exchange stride: an odd number of 16-byte words
+    static constexpr int GS = (M * M) | 1;                        // stride of a problem's matrix
+    static constexpr int CS = 2 * (M / 2 + 1);                    // rotations of a Jacobi stage
+    static constexpr int R = C <= 5 ? 2 : 1;                      // gradient solves run side by side
+    static constexpr int kVec = 3 * M + 9 * C + C * C + 6 * C;    // per problem: b, MJ column, work, Z, B, sigma
 };
 
-__host__ __device__ inline size_t env_doubles(int C, int NV)
+__host__ __device__ constexpr int odd(int n) { return n | 1; }
+
+// staging of one problem while G is formed: J and M^-1 J^T (M rows) and M^-1 (nv rows), rows padded
+template <int C>
+__host__ __device__ inline size_t stage_doubles(int nv)
 {
-    const size_t M = 3 * (size_t)C;
-    return M * NV * 2 + (size_t)NV * NV + M * M * 2 + (size_t)C * NV + 2 * (size_t)NV + 24 * M + 10 * (size_t)C +
-           36 * (size_t)C + 2 * (size_t)C * C + C;
+    return (size_t)(2 * Dim<C>::M + nv) * odd(nv);
 }
-__host__ __device__ inline size_t env_bytes(int C, int NV)
+template <int C>
+__host__ __device__ inline size_t work_doubles(int nv)
 {
-    return env_doubles(C, NV) * 8 + (size_t)C * 4 + 16;
+    const size_t a = (size_t)Dim<C>::PW * Dim<C>::GS, b = stage_doubles<C>(nv);
+    return (a > b ? a : b) + 1;
+}
+template <int C>
+inline size_t smem_bytes(int nv)
+{
+    using D = Dim<C>;
+    return 8 * (2 * (size_t)D::PW * D::XS * D::R + (size_t)D::PW * (D::GS + D::CS + D::kVec) + work_doubles<C>(nv));
 }
 
-__device__ inline Env carve(double *base, int C, int NV)
+// f_proj (NB:113-126); icm = 1 / (1 + mu^2)
+__device__ __forceinline__ void proj3(const double z[3], double mu, double icm, double out[3])
 {
-    Env E;
-    E.C = C;
-    E.NV = NV;
-    E.M = 3 * C;
-    const int M = E.M;
-    double *p = base;
-    auto take = [&](size_t n) {
-        double *q = p;
-        p += n;
-        return q;
-    };
-    E.J = take((size_t)M * NV);
-    E.MJ = take((size_t)M * NV);
-    E.Mi = take((size_t)NV * NV);
-    E.G = take((size_t)M * M);
-    E.A = take((size_t)M * M);
-    E.yt = take((size_t)C * NV);
-    E.wv = take(NV);
-    E.vf = take(NV);
-    double **vecs[] = {&E.bb, &E.x, &E.zv, &E.gam, &E.r, &E.zz, &E.pv, &E.Ap, &E.rhs, &E.tmp, &E.tmp2, &E.u,
-                       &E.pinh, &E.dbv, &E.ZtHp, &E.yv, &E.dlam, &E.Dv, &E.what, &E.bw, &E.ev};
-    for (double **v : vecs) *v = take(M);
-    take(3 * (size_t)M);  // (24 vectors of M reserved)
-    double **cvec[] = {&E.mu, &E.s, &E.eta, &E.rhoc, &E.slipf, &E.sig, &E.sigo, &E.siga, &E.res, &E.gnorm};
-    for (double **v : cvec) *v = take(C);
-    E.Gd = take(9 * (size_t)C);
-    E.Pj = take(9 * (size_t)C);
-    E.Zm = take(9 * (size_t)C);
-    E.Ps = take(9 * (size_t)C);
-    E.Bm = take((size_t)C * C);
-    E.Aw = take((size_t)C * C);
-    E.rw = take(C);
-    E.sidx = reinterpret_cast<int *>(p);
-    E.kap = 0.0;
-    E.rho = 0.0;
-    E.mask = 1;
-    E.nslip = 0;
-    return E;
-}
-
-__device__ __forceinline__ int lane_id() { return (int)(threadIdx.x & 31); }
-__device__ __forceinline__ double warp_max(double v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-
-// f_proj (NB:113-126)
-__device__ __forceinline__ void proj3(const double z[3], double mu, double out[3])
-{
-    const double zn = z[0], zt = sqrt(z[1] * z[1] + z[2] * z[2]);
+    const double zn = z[0], zt = sqrt(fma(z[1], z[1], z[2] * z[2]));
     if (zt <= mu * zn) {
         out[0] = z[0];
         out[1] = z[1];
@@ -120,7 +92,7 @@ __device__ __forceinline__ void proj3(const double z[3], double mu, double out[3
     } else if (mu * zt <= -zn) {
         out[0] = out[1] = out[2] = 0.0;
     } else {
-        const double s = (zn + mu * zt) / (1.0 + mu * mu);
+        const double s = fma(mu, zt, zn) * icm;
         const double f = mu * s / zt;
         out[0] = s;
         out[1] = f * z[1];
@@ -136,6 +108,7 @@ __device__ inline void inv3(const double a[9], double o[9])
     const double c20 = a[3] * a[7] - a[4] * a[6], c21 = a[1] * a[6] - a[0] * a[7], c22 = a[0] * a[4] - a[1] * a[3];
     const double det = a[0] * c00 + a[1] * c10 + a[2] * c20;
     const double adj[9] = {c00, c01, c02, c10, c11, c12, c20, c21, c22};
+#pragma unroll
     for (int i = 0; i < 9; ++i) o[i] = det != 0.0 ? adj[i] / det : 0.0;
 }
 
@@ -150,6 +123,7 @@ __device__ inline double eigmax3(const double A[9])
         const double p = sqrt(p2 / 6.0);
         if (p > 1.0e-300) {
             double Bm[9];
+#pragma unroll
             for (int i = 0; i < 9; ++i) Bm[i] = (A[i] - ((i % 4) == 0 ? q : 0.0)) / p;
             const double det = Bm[0] * (Bm[4] * Bm[8] - Bm[5] * Bm[7]) - Bm[1] * (Bm[3] * Bm[8] - Bm[5] * Bm[6]) +
                                Bm[2] * (Bm[3] * Bm[7] - Bm[4] * Bm[6]);
@@ -160,609 +134,826 @@ __device__ inline double eigmax3(const double A[9])
     return out;
 }
 
-// the matrix-free product (k_scale, k_jt, k_mscat, k_acc2w, k_gath): xout = G xin + (eta + rho') xin.
-// Lane k (< nv) owns row k of M^-1: it forms every contact's M^-1 (J^T x)_c entry k with the
-// contacts' sums interleaved (independent chains), rounds each at the scale and adds them in its
-// own int64 register -- exact, so no atomics and no order dependence.  The scale is a power of
-// two, so acc / scale is the exact product acc * 2^-e.
-template <int kC>
-__device__ void matvec(Env &E, const double *xin, double *xout, bool use_rho)
+// one warp's view of its shared memory; g is the problem (lane group) of this lane
+template <int C>
+struct Env {
+    using D = Dim<C>;
+    int ln, g, c;       // lane, problem within the warp, contact
+    bool on;            // this lane owns a contact (c < C)
+    int turn;           // which exchange buffer is next
+    double *xch;        // two buffers of PW x XS x R
+    double *G, *A;      // the problem's G; scratch of the same shape (the spectrum, the Cholesky factor)
+    double *cs;         // the stage's rotations
+    double *bb, *mjc, *bw, *Z, *Bm, *a, *sg;  // b, (M^-1 J^T) column, work, projectors, B, a (2 x C), sigma (2 x C)
+    double *stage;      // the whole warp's staging area (A's storage)
+};
+
+template <int C>
+__device__ inline Env<C> carve(double *p, int nv)
 {
-    const int ln = lane_id(), C = E.C, NV = E.NV, M = E.M;
-    double m = ln < M ? fabs(xin[ln]) : 0.0;
-    m = warp_max(m);
-    const double t = E.kap * m;
-    double scal = 1.0, inv = 1.0;
-    if (t > 0.0) {
-        int e = ilogb(kScaleBound / t);  // floor(log2(2^52 / t)), exactly
-        e = e < -1000 ? -1000 : (e > 1000 ? 1000 : e);
-        scal = ldexp(1.0, e);
-        inv = ldexp(1.0, -e);
-    }
-    if (ln < NV) {
-#pragma unroll
-        for (int c = 0; c < kC; ++c) {
-            const double *jr = E.J + (size_t)(3 * c) * NV + ln;
-            E.yt[c * NV + ln] = jr[0] * xin[3 * c] + jr[NV] * xin[3 * c + 1] + jr[2 * NV] * xin[3 * c + 2];
-        }
-    }
-    __syncwarp();
-    if (ln < NV) {
-        double sc[kC];
-#pragma unroll
-        for (int c = 0; c < kC; ++c) sc[c] = 0.0;
-        const double *mrow = E.Mi + (size_t)ln * NV;
-        for (int l = 0; l < NV; ++l) {
-            const double ml = mrow[l];
-#pragma unroll
-            for (int c = 0; c < kC; ++c) sc[c] = sc[c] + ml * E.yt[c * NV + l];
-        }
-        long long acc = 0;
-#pragma unroll
-        for (int c = 0; c < kC; ++c) acc += llround(sc[c] * scal);
-        E.wv[ln] = (double)acc * inv;
-    }
-    __syncwarp();
-    const double rr = use_rho ? E.rho : 0.0;
-    if (ln < M) {
-        double u = 0.0;
-        const double *jrow = E.J + (size_t)ln * NV;
-        for (int k = 0; k < NV; ++k) u = u + jrow[k] * E.wv[k];
-        xout[ln] = u + (E.eta[ln / 3] + rr) * xin[ln];
-    }
-    __syncwarp();
+    using D = Dim<C>;
+    Env<C> E;
+    E.ln = (int)(threadIdx.x & 31);
+    E.g = E.ln / D::L;
+    E.c = E.ln % D::L;
+    E.on = E.c < C;
+    E.turn = 0;
+    E.xch = p;
+    p += 2 * D::PW * D::XS * D::R;
+    E.stage = p;
+    E.A = p + (size_t)E.g * D::GS;
+    p += work_doubles<C>(nv);
+    E.G = p + (size_t)E.g * D::GS;
+    p += (size_t)D::PW * D::GS;
+    E.cs = p + (size_t)E.g * D::CS;
+    p += (size_t)D::PW * D::CS;
+    p += (size_t)E.g * D::kVec;
+    E.bb = p;
+    E.mjc = p + D::M;
+    E.bw = p + 2 * D::M;
+    E.Z = p + 3 * D::M;
+    E.Bm = E.Z + 9 * C;
+    E.a = E.Bm + C * C;
+    E.sg = E.a + 3 * C;
+    return E;
 }
 
-// k_dot (NB:408-416): the products lane by lane, summed by a butterfly; IEEE addition is
-// commutative, so every lane ends with the same bits
-__device__ __forceinline__ double dot(const Env &E, const double *a, const double *b)
+// sum over the problem's lanes: a butterfly, the same bits on every lane (IEEE addition commutes)
+template <int L>
+__device__ __forceinline__ double gsum(double s)
 {
-    const int ln = lane_id();
-    double s = ln < E.M ? a[ln] * b[ln] : 0.0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s = s + __shfl_xor_sync(0xffffffffu, s, o);
+    for (int o = L / 2; o > 0; o >>= 1) s = s + __shfl_xor_sync(kAll, s, o);
     return s;
 }
-
-// k_papply: z = P r per contact
-__device__ __forceinline__ void papply(const Env &E, const double *P, const double *r, double *z)
+__device__ __forceinline__ double dot3(const double a[3], const double b[3])
 {
-    for (int i = lane_id(); i < E.M; i += 32) {
-        const int c = i / 3, row = i - 3 * c;
-        const double *p = P + 9 * c + 3 * row;
-        z[i] = p[0] * r[3 * c] + p[1] * r[3 * c + 1] + p[2] * r[3 * c + 2];
-    }
-    __syncwarp();
+    return fma(a[2], b[2], fma(a[1], b[1], a[0] * b[0]));
 }
 
-// the Schur operator of the fixed-branch system (NB:1040-1043): yout = Z^T G Z y + D y
-template <int kC>
-__device__ void sopv(Env &E, const double *y, double *yout)
+// y[k] = rows x for N vectors at once: the lanes pass their three entries through shared memory
+// (two buffers in turn, so one __syncwarp an exchange: a lane writes a buffer again only after
+// the barrier that follows its last reads of it) and each forms its contact's three rows in two
+// interleaved sums a row
+template <int C, int N>
+__device__ __forceinline__ void rows_times(Env<C> &E, const double (&g)[3][3 * C], const double (&x)[N][3],
+                                           double (&y)[N][3])
 {
-    const int ln = lane_id();
-    for (int i = ln; i < E.M; i += 32) {
-        const int c = i / 3, row = i - 3 * c;
-        const double *z = E.Zm + 9 * c + 3 * row;
-        E.tmp[i] = z[0] * y[3 * c] + z[1] * y[3 * c + 1] + z[2] * y[3 * c + 2];
+    using D = Dim<C>;
+    constexpr int NS = D::PW * D::XS;  // from one vector of the exchange to the next
+    double *buf = E.xch + (size_t)E.turn * D::R * NS + E.g * D::XS;
+    E.turn ^= 1;
+    if (E.on) {
+#pragma unroll
+        for (int n = 0; n < N; ++n)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) buf[n * NS + 3 * E.c + k] = x[n][k];
     }
     __syncwarp();
-    matvec<kC>(E, E.tmp, E.tmp2, false);
-    for (int i = ln; i < E.M; i += 32) {
-        const int c = i / 3, col = i - 3 * c;
-        const double *z = E.Zm + 9 * c;
-        const double t = z[col] * E.tmp2[3 * c] + z[3 + col] * E.tmp2[3 * c + 1] + z[6 + col] * E.tmp2[3 * c + 2];
-        yout[i] = t + E.Dv[i] * y[i];
-    }
-    __syncwarp();
-}
-
-enum Op { kOpAdmm = 0, kOpSchur = 1 };
-
-// _pcg (NB:1048-1073); the x update skips a frozen problem when use_mask
-template <int kC>
-__device__ void pcg(Env &E, const double *rhs, double *x, int n_it, Op op, const double *P, bool warm_zero,
-                    bool use_mask)
-{
-    const int ln = lane_id(), M = E.M;
-    auto apply = [&](const double *v, double *o) {
-        if (op == kOpAdmm) matvec<kC>(E, v, o, true);
-        else sopv<kC>(E, v, o);
-    };
-    if (warm_zero) {
-        for (int i = ln; i < M; i += 32) {
-            x[i] = 0.0;
-            E.r[i] = rhs[i];
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+        double s0[3], s1[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) s0[k] = s1[k] = 0.0;
+        const double2 *q = reinterpret_cast<const double2 *>(buf + n * NS);
+#pragma unroll
+        for (int j = 0; j < D::M / 2; ++j) {
+            const double2 v = q[j];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                s0[k] = fma(g[k][2 * j], v.x, s0[k]);
+                s1[k] = fma(g[k][2 * j + 1], v.y, s1[k]);
+            }
         }
-        __syncwarp();
-    } else {
-        apply(x, E.Ap);
-        for (int i = ln; i < M; i += 32) E.r[i] = rhs[i] - E.Ap[i];
-        __syncwarp();
+        if (D::M & 1) {
+            const double v = buf[n * NS + D::M - 1];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) s0[k] = fma(g[k][D::M - 1], v, s0[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) y[n][k] = s0[k] + s1[k];
     }
-    papply(E, P, E.r, E.zz);
-    for (int i = ln; i < M; i += 32) E.pv[i] = E.zz[i];
-    __syncwarp();
-    double s0 = dot(E, E.r, E.zz);
-    const bool upd = !use_mask || E.mask != 0;
+}
+
+__device__ __forceinline__ void apply3(const double P[9], const double r[3], double z[3])
+{
+#pragma unroll
+    for (int k = 0; k < 3; ++k) z[k] = fma(P[3 * k + 2], r[2], fma(P[3 * k + 1], r[1], P[3 * k] * r[0]));
+}
+
+// _pcg (NB:1048-1073) on N right-hand sides at once: the operator is rows + diag(d), the
+// preconditioner the lane's 3x3 block P; x is updated where `upd`.  beta = s3 / s0 by the
+// reciprocal of s0, which is formed beside the product instead of after the dot product; below
+// 1e-290, where the reciprocal would overflow, by the quotient itself.
+template <int C, int N>
+__device__ __forceinline__ void pcg(Env<C> &E, const double (&g)[3][3 * C], const double (&d)[3], const double P[9],
+                                    const double (&rhs)[N][3], double (&x)[N][3], int n_it, bool zero, bool upd)
+{
+    using D = Dim<C>;
+    double r[N][3], p[N][3], Ap[N][3], s0[N];
+    if (zero) {
+#pragma unroll
+        for (int n = 0; n < N; ++n)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                x[n][k] = 0.0;
+                r[n][k] = rhs[n][k];
+            }
+    } else {
+        rows_times<C, N>(E, g, x, Ap);
+#pragma unroll
+        for (int n = 0; n < N; ++n)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) r[n][k] = rhs[n][k] - fma(d[k], x[n][k], Ap[n][k]);
+    }
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+        apply3(P, r[n], p[n]);
+        s0[n] = gsum<D::L>(dot3(r[n], p[n]));
+    }
     for (int it = 0; it < n_it; ++it) {
-        apply(E.pv, E.Ap);
-        const double s1 = dot(E, E.pv, E.Ap);
-        const double s2 = (s1 > 0.0 || s1 < 0.0) ? s0 / s1 : 0.0;
-        for (int i = ln; i < M; i += 32) {
-            if (upd) x[i] = x[i] + 1.0 * s2 * E.pv[i];
-            E.r[i] = E.r[i] + -1.0 * s2 * E.Ap[i];
+        rows_times<C, N>(E, g, p, Ap);
+        double s1[N], i0[N];
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+            i0[n] = 1.0 / s0[n];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) Ap[n][k] = fma(d[k], p[n][k], Ap[n][k]);
+            s1[n] = gsum<D::L>(dot3(p[n], Ap[n]));
         }
-        __syncwarp();
-        papply(E, P, E.r, E.zz);
-        const double s3 = dot(E, E.r, E.zz);
-        const double s4 = (s0 > 0.0 || s0 < 0.0) ? s3 / s0 : 0.0;
-        for (int i = ln; i < M; i += 32) E.pv[i] = E.zz[i] + s4 * E.pv[i];
-        __syncwarp();
-        s0 = s3;
-    }
-}
-
-// one ADMM iteration (NB:1075-1082)
-template <int kC>
-__device__ void admm_iter(Env &E, int cg_iters)
-{
-    const int ln = lane_id(), M = E.M;
-    for (int i = ln; i < M; i += 32) {
-        const int c = i / 3;
-        const double g = E.bb[i] + ((i - 3 * c) == 0 ? E.mu[c] * E.s[c] : 0.0);
-        E.rhs[i] = -((g + E.gam[i]) - E.rho * E.zv[i]);
-    }
-    __syncwarp();
-    pcg<kC>(E, E.rhs, E.x, cg_iters, kOpAdmm, E.Pj, false, true);
-    if (E.mask != 0) {
-        for (int c = ln; c < E.C; c += 32) {
-            double v[3], z[3];
-            for (int k = 0; k < 3; ++k) v[k] = E.x[3 * c + k] + E.gam[3 * c + k] / E.rho;
-            proj3(v, E.mu[c], z);
-            for (int k = 0; k < 3; ++k) E.zv[3 * c + k] = z[k];
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+            const double s2 = (s1[n] > 0.0 || s1[n] < 0.0) ? s0[n] / s1[n] : 0.0;
+            double z[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                if (upd) x[n][k] = fma(s2, p[n][k], x[n][k]);
+                r[n][k] = fma(-s2, Ap[n][k], r[n][k]);
+            }
+            apply3(P, r[n], z);
+            const double s3 = gsum<D::L>(dot3(r[n], z));
+            double s4 = s3 * i0[n];
+            if (!(fabs(s0[n]) > 1e-290)) s4 = (s0[n] > 0.0 || s0[n] < 0.0) ? s3 / s0[n] : 0.0;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) p[n][k] = fma(s4, p[n][k], z[k]);
+            s0[n] = s3;
         }
-        __syncwarp();
-        for (int i = ln; i < M; i += 32) E.gam[i] = E.gam[i] + E.rho * (E.x[i] - E.zv[i]);
-        __syncwarp();
     }
 }
 
-// the Cadoux refresh, the natural residual and the mask (NB:1084-1092, 498-543)
-template <int kC>
-__device__ double refresh(Env &E, double tol, bool desax)
+// G's eigenvalues into the diagonal of E.A (k_jacobi): `sweeps` cyclic Jacobi sweeps in the
+// row-cyclic pair order (0,1), (0,2), ..., (M-2, M-1).  Rotations on disjoint pairs commute, and
+// in that order the pair (p, q) of sweep s only waits for pairs of smaller p + q + s M: stage t
+// therefore runs every pair with p + q = t (mod M) at once, two sweeps overlapping, and M stages
+// do a sweep's work where the pairs one by one are M (M - 1) / 2 steps.  A stage is a rotation
+// per pair (spread over the problem's lanes), then the 2x2 blocks of the pairs' rows and columns,
+// each one lane's.  It ends early when a whole sweep met no off-diagonal entry above 1e-17 of its
+// diagonal's geometric mean: no eigenvalue can move by a rounding any more.
+template <int C>
+__device__ void spectrum(Env<C> &E, int sweeps)
 {
-    const int ln = lane_id();
-    matvec<kC>(E, E.zv, E.tmp2, false);
-    for (int i = ln; i < E.M; i += 32) E.u[i] = E.tmp2[i] + E.bb[i];
-    __syncwarp();
-    for (int c = ln; c < E.C; c += 32) {
-        const double *uu = E.u + 3 * c;
-        const double ut = sqrt(uu[1] * uu[1] + uu[2] * uu[2]);
-        E.s[c] = ut;
-        double w[3] = {uu[0], uu[1], uu[2]};
-        if (desax) w[0] = uu[0] + E.mu[c] * ut;
-        double q[3], pr[3];
-        for (int k = 0; k < 3; ++k) q[k] = E.zv[3 * c + k] - E.rhoc[c] * w[k];
-        proj3(q, E.mu[c], pr);
-        const double d0 = fabs(E.zv[3 * c] - pr[0]), d1 = fabs(E.zv[3 * c + 1] - pr[1]),
-                     d2 = fabs(E.zv[3 * c + 2] - pr[2]);
-        E.res[c] = fmax(d0, fmax(d1, d2));
-    }
-    __syncwarp();
-    double m = 0.0;
-    for (int c = 0; c < E.C; ++c) {  // NaN-propagating maximum (k_resmax)
-        const double v = E.res[c];
-        if (v != v) m = v;
-        else if (v > m) m = v;
-    }
-    if (E.mask == 1 && m < tol) E.mask = 0;
-    return m;
-}
-
-// set-up of one problem (NB:974-1000, 1013-1022, k_pjac)
-__device__ void setup(Env &E, const b2c_admm &P, const b2c_admm_params &prm, int e)
-{
-    const int ln = lane_id(), C = E.C, NV = E.NV, M = E.M;
-    const double *Jg = P.J + (size_t)e * M * NV, *Mg = P.Minv + (size_t)e * NV * NV, *vg = P.v_free + (size_t)e * NV;
-    for (int i = ln; i < M * NV; i += 32) E.J[i] = Jg[i];
-    for (int i = ln; i < NV * NV; i += 32) E.Mi[i] = Mg[i];
-    for (int i = ln; i < NV; i += 32) E.vf[i] = vg[i];
-    for (int c = ln; c < C; c += 32) E.mu[c] = P.mu[(size_t)e * C + c];
-    __syncwarp();
-    for (int i = ln; i < M; i += 32) {
-        double s = 0.0;
-        for (int k = 0; k < NV; ++k) s = s + E.J[i * NV + k] * E.vf[k];
-        E.bb[i] = P.b_in ? P.b_in[(size_t)e * M + i] : s;
-    }
-    // kappa = C max_i sum_l |M^-1_il| max_(c,k) sum_r |J_(3c+r)k| + 1e-300
-    double m1 = 0.0, m2 = 0.0;
-    for (int i = ln; i < NV; i += 32) {
-        double s = 0.0;
-        for (int l = 0; l < NV; ++l) s = s + fabs(E.Mi[i * NV + l]);
-        m1 = fmax(m1, s);
-    }
-    for (int q = ln; q < C * NV; q += 32) {
-        const int c = q / NV, k = q - c * NV;
-        m2 = fmax(m2, fabs(E.J[(3 * c) * NV + k]) + fabs(E.J[(3 * c + 1) * NV + k]) + fabs(E.J[(3 * c + 2) * NV + k]));
-    }
-    m1 = warp_max(m1);
-    m2 = warp_max(m2);
-    E.kap = (double)C * m1 * m2 + 1e-300;
-    // M^-1 J^T (k_mj) and G = J M^-1 J^T (k_gdense)
-    for (int q = ln; q < M * NV; q += 32) {
-        const int i = q / NV, k = q - i * NV;
-        double s = 0.0;
-        for (int l = 0; l < NV; ++l) s = s + E.Mi[k * NV + l] * E.J[i * NV + l];
-        E.MJ[q] = s;
-    }
-    __syncwarp();
-    for (int q = ln; q < M * M; q += 32) {
-        const int i = q / M, j = q - i * M;
-        double s = 0.0;
-        for (int k = 0; k < NV; ++k) s = s + E.J[i * NV + k] * E.MJ[j * NV + k];
-        E.G[q] = s;
-        E.A[q] = s;
-    }
-    __syncwarp();
-    // spectrum: cyclic Jacobi in the fixed pair order (k_jacobi); lane k updates row / column k
-    for (int sw = 0; sw < prm.jacobi_sweeps; ++sw)
-        for (int p = 0; p < M - 1; ++p)
-            for (int q = p + 1; q < M; ++q) {
-                const double apq = E.A[p * M + q];
+    using D = Dim<C>;
+    constexpr int M = D::M;
+    double *A = E.A, *cs = E.cs;
+    bool big = false;
+    for (int t = 1; t <= sweeps * M + M - 3; ++t) {
+        const int r = t % M, s = t / M;
+        const int n1 = r / 2 + 1, K = n1 + (r + M) / 2 - r;  // pairs with p + q = r, and with p + q = r + M
+        for (int k = E.c; k < K; k += D::L) {
+            const int p = k < n1 ? k : r + 1 + (k - n1), q = k < n1 ? r - p : r + M - p;
+            const int sw = k < n1 ? s : s - 1;
+            double c = 1.0, sn = 0.0;
+            if (p != q && sw >= 0 && sw < sweeps) {
+                const double apq = A[p * M + q], app = A[p * M + p], aqq = A[q * M + q];
                 if (apq > kTiny || apq < -kTiny) {
-                    const double app = E.A[p * M + p], aqq = E.A[q * M + q];
+                    if (apq * apq > 1e-34 * fabs(app * aqq)) big = true;
                     const double th = (aqq - app) / (2.0 * apq);
-                    double t = 1.0 / (fabs(th) + sqrt(th * th + 1.0));
-                    if (th < 0.0) t = -t;
-                    const double c = 1.0 / sqrt(t * t + 1.0), sn = t * c;
-                    __syncwarp();
-                    for (int k = ln; k < M; k += 32) {
-                        const double akp = E.A[k * M + p], akq = E.A[k * M + q];
-                        E.A[k * M + p] = c * akp - sn * akq;
-                        E.A[k * M + q] = sn * akp + c * akq;
-                    }
-                    __syncwarp();
-                    for (int k = ln; k < M; k += 32) {
-                        const double apk = E.A[p * M + k], aqk = E.A[q * M + k];
-                        E.A[p * M + k] = c * apk - sn * aqk;
-                        E.A[q * M + k] = sn * apk + c * aqk;
-                    }
-                    __syncwarp();
+                    double tt = 1.0 / (fabs(th) + sqrt(fma(th, th, 1.0)));
+                    if (th < 0.0) tt = -tt;
+                    c = 1.0 / sqrt(fma(tt, tt, 1.0));
+                    sn = tt * c;
                 }
             }
-    for (int i = ln; i < M; i += 32) E.ev[i] = E.A[i * M + i];
-    // diagonal blocks, their largest eigenvalue, eta, the per-contact step (k_gd3, k_eta)
-    for (int c = ln; c < C; c += 32) {
-        double W[9];
-        for (int i = 0; i < 3; ++i)
-            for (int j = 0; j < 3; ++j) W[3 * i + j] = E.G[(3 * c + i) * M + 3 * c + j];
-        for (int i = 0; i < 9; ++i) E.Gd[9 * c + i] = W[i];
-        const double gn = eigmax3(W);
-        E.gnorm[c] = gn;
-        E.eta[c] = prm.alpha_eta * gn;
-        const double s = gn + E.eta[c];
-        E.rhoc[c] = s > 0.0 ? 1.0 / s : 1.0;
-    }
-    __syncwarp();
-    // the regime (k_bilat): Cholesky of G with floored pivots, then -G^-1 b against the cones;
-    // run by lane 0 (a 3 nc x 3 nc factorisation)
-    int bind = 0;
-    if (prm.rho_mode == B2C_ADMM_RHO_REGIME) {
-        if (ln == 0) {
-            for (int i = 0; i < M * M; ++i) E.A[i] = E.G[i];
-            for (int k = 0; k < M; ++k) {
-                double d = E.A[k * M + k];
-                for (int j = 0; j < k; ++j) d = d - E.A[k * M + j] * E.A[k * M + j];
-                if (d < kTiny) d = kTiny;
-                d = sqrt(d);
-                E.A[k * M + k] = d;
-                for (int i = k + 1; i < M; ++i) {
-                    double s = E.A[i * M + k];
-                    for (int j = 0; j < k; ++j) s = s - E.A[i * M + j] * E.A[k * M + j];
-                    E.A[i * M + k] = s / d;
+            cs[2 * k] = c;
+            cs[2 * k + 1] = sn;
+        }
+        __syncwarp();
+        for (int P = 0; P < K; ++P) {
+            const int p = P < n1 ? P : r + 1 + (P - n1), q = P < n1 ? r - p : r + M - p;
+            const double cp = cs[2 * P], sp = cs[2 * P + 1];
+            for (int Q = E.c; Q < K; Q += D::L) {
+                const int u = Q < n1 ? Q : r + 1 + (Q - n1), v = Q < n1 ? r - u : r + M - u;
+                const double cq = cs[2 * Q], sq = cs[2 * Q + 1];
+                const double b00 = A[p * M + u], b01 = A[p * M + v], b10 = A[q * M + u], b11 = A[q * M + v];
+                const double e00 = cq * b00 - sq * b01, e01 = sq * b00 + cq * b01;
+                const double e10 = cq * b10 - sq * b11, e11 = sq * b10 + cq * b11;
+                A[p * M + u] = cp * e00 - sp * e10;
+                if (u != v) A[p * M + v] = cp * e01 - sp * e11;
+                if (p != q) {
+                    A[q * M + u] = sp * e00 + cp * e10;
+                    if (u != v) A[q * M + v] = sp * e01 + cp * e11;
                 }
             }
-            for (int i = 0; i < M; ++i) {
-                double s = -E.bb[i];
-                for (int j = 0; j < i; ++j) s = s - E.A[i * M + j] * E.bw[j];
-                E.bw[i] = s / E.A[i * M + i];
-            }
-            for (int ii = 0; ii < M; ++ii) {
-                const int i = M - 1 - ii;
-                double s = E.bw[i];
-                for (int j = i + 1; j < M; ++j) s = s - E.A[j * M + i] * E.bw[j];
-                E.bw[i] = s / E.A[i * M + i];
-            }
-            for (int c = 0; c < C; ++c) {
-                const double lnrm = E.bw[3 * c], lt = sqrt(E.bw[3 * c + 1] * E.bw[3 * c + 1] + E.bw[3 * c + 2] * E.bw[3 * c + 2]);
-                if (lnrm <= 0.0 || lt > E.mu[c] * lnrm) bind = 1;
-            }
         }
-        bind = __shfl_sync(0xffffffffu, bind, 0);
-    }
-    // rho (k_rho): sqrt(lmin+ lmax) | lmin+ | lmax | the regime's choice
-    double mx = -1.0e300;
-    for (int i = 0; i < M; ++i) mx = fmax(mx, E.ev[i]);
-    const double thr = 1e-12 * mx;
-    double mn = mx;
-    for (int i = 0; i < M; ++i) {
-        const double v = E.ev[i];
-        if (v > thr && v < mn) mn = v;
-    }
-    double rho = sqrt(mn * mx);
-    if (prm.rho_mode == B2C_ADMM_RHO_LMIN) rho = mn;
-    if (prm.rho_mode == B2C_ADMM_RHO_LMAX) rho = mx;
-    if (prm.rho_mode == B2C_ADMM_RHO_REGIME) rho = bind ? mx : mn;
-    if (prm.rho_mode == B2C_ADMM_RHO_GIVEN) rho = P.rho[e];
-    E.rho = rho;
-    // block-Jacobi preconditioner (k_pjac) and the reset (NB:1100-1110)
-    for (int c = ln; c < C; c += 32) {
-        double W[9];
-        const double sh = E.eta[c] + rho;
-        for (int i = 0; i < 9; ++i) W[i] = E.Gd[9 * c + i] + ((i % 4) == 0 ? sh : 0.0);
-        inv3(W, E.Pj + 9 * c);
-    }
-    for (int i = ln; i < M; i += 32) {
-        E.gam[i] = 0.0;
-        E.zv[i] = 0.0;
-        E.x[i] = 0.0;
-        E.u[i] = 0.0;
-    }
-    for (int c = ln; c < C; c += 32) E.s[c] = 0.0;
-    E.mask = 1;
-    __syncwarp();
-}
-
-// the active set (k_lamscale, k_active, k_slipidx, k_sjac: NB:546-627), from lam = zv and u
-__device__ void build_active(Env &E, double tol_lam, double tol_rel)
-{
-    const int ln = lane_id(), C = E.C;
-    double lsc = 1.0e-30;
-    for (int i = 0; i < E.M; ++i) lsc = fmax(lsc, fabs(E.zv[i]));
-    for (int c = ln; c < C; c += 32) {
-        const double *L = E.zv + 3 * c;
-        const double lnrm = L[0], lt = sqrt(L[1] * L[1] + L[2] * L[2]);
-        double Z[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-        double D[3] = {0, 0, 0}, wh[3] = {0, 0, 0}, sf = 0.0;
-        const double mu = E.mu[c];
-        if (lnrm <= tol_lam + tol_rel * lsc) {  // open
-            D[0] = D[1] = D[2] = 1.0;
-        } else if (lt >= mu * lnrm * (1.0 - tol_rel) - tol_lam) {  // slip
-            const double w1 = E.u[3 * c + 1], w2 = E.u[3 * c + 2];
-            double nw = sqrt(w1 * w1 + w2 * w2);
-            if (nw < 1.0e-300) nw = 1.0e-300;
-            const double h1 = w1 / nw, h2 = w2 / nw;
-            Z[0] = 1.0;
-            Z[3] = -mu * h1;
-            Z[6] = -mu * h2;
-            Z[4] = -h2;
-            Z[7] = h1;
-            D[1] = nw / fmax(mu * lnrm, 1.0e-300);
-            D[2] = 1.0;
-            sf = 1.0;
-            wh[1] = h1;
-            wh[2] = h2;
-        } else {  // stick
-            Z[0] = Z[4] = Z[8] = 1.0;
-        }
-        for (int i = 0; i < 9; ++i) E.Zm[9 * c + i] = Z[i];
-        for (int k = 0; k < 3; ++k) {
-            E.Dv[3 * c + k] = D[k];
-            E.what[3 * c + k] = wh[k];
-        }
-        E.slipf[c] = sf;
-        // Schur preconditioner: (Z^T (Gd + eta I) Z + diag D)^-1
-        double Q[9], T[9], S[9];
-        for (int i = 0; i < 9; ++i) Q[i] = E.Gd[9 * c + i] + ((i % 4) == 0 ? E.eta[c] : 0.0);
-        for (int i = 0; i < 3; ++i)
-            for (int j = 0; j < 3; ++j) {
-                double s = 0.0;
-                for (int k = 0; k < 3; ++k) s = s + Z[3 * k + i] * Q[3 * k + j];
-                T[3 * i + j] = s;
-            }
-        for (int i = 0; i < 3; ++i)
-            for (int j = 0; j < 3; ++j) {
-                double s = 0.0;
-                for (int k = 0; k < 3; ++k) s = s + T[3 * i + k] * Z[3 * k + j];
-                S[3 * i + j] = s;
-            }
-        S[0] += D[0];
-        S[4] += D[1];
-        S[8] += D[2];
-        inv3(S, E.Ps + 9 * c);
-    }
-    __syncwarp();
-    int n = 0;
-    for (int c = 0; c < C; ++c)
-        if (E.slipf[c] > 0.5) {
-            if (ln == 0) E.sidx[n] = c;
-            ++n;
-        }
-    for (int c = n + ln; c < C; c += 32) E.sidx[c] = -1;
-    E.nslip = n;
-    __syncwarp();
-}
-
-// one application of the affine sigma map (NB:1162-1170)
-template <int kC>
-__device__ void grad_once(Env &E, int cg)
-{
-    const int ln = lane_id(), M = E.M;
-    for (int i = ln; i < M; i += 32) {
-        const int c = i / 3;
-        double v = -E.ZtHp[i];
-        if (E.slipf[c] > 0.5 && i == 3 * c) v = v - E.mu[c] * E.sig[c];
-        E.rhs[i] = v;
-    }
-    __syncwarp();
-    pcg<kC>(E, E.rhs, E.yv, cg, kOpSchur, E.Ps, true, false);
-    for (int i = ln; i < M; i += 32) {
-        const int c = i / 3, row = i - 3 * c;
-        const double *z = E.Zm + 9 * c + 3 * row;
-        E.dlam[i] = (z[0] * E.yv[3 * c] + z[1] * E.yv[3 * c + 1] + z[2] * E.yv[3 * c + 2]) + E.pinh[i];
-    }
-    __syncwarp();
-    matvec<kC>(E, E.dlam, E.tmp2, false);
-    for (int c = ln; c < E.C; c += 32)
-        E.sigo[c] = E.slipf[c] > 0.5 ? E.what[3 * c + 1] * (E.tmp2[3 * c + 1] + E.dbv[3 * c + 1]) +
-                                            E.what[3 * c + 2] * (E.tmp2[3 * c + 2] + E.dbv[3 * c + 2])
-                                      : 0.0;
-    __syncwarp();
-}
-
-// grad_affine (NB:1172-1186): dlam for the current (pinh, dbv)
-template <int kC>
-__device__ void grad_affine(Env &E, int n_calls, int cg)
-{
-    const int ln = lane_id(), C = E.C, M = E.M;
-    const int K = n_calls - 2;
-    matvec<kC>(E, E.pinh, E.tmp, false);
-    for (int i = ln; i < M; i += 32) E.tmp2[i] = E.tmp[i] + E.dbv[i];
-    __syncwarp();
-    for (int i = ln; i < M; i += 32) {
-        const int c = i / 3, col = i - 3 * c;
-        const double *z = E.Zm + 9 * c;
-        E.ZtHp[i] = z[col] * E.tmp2[3 * c] + z[3 + col] * E.tmp2[3 * c + 1] + z[6 + col] * E.tmp2[3 * c + 2];
-    }
-    for (int c = ln; c < C; c += 32) E.sig[c] = 0.0;
-    __syncwarp();
-    grad_once<kC>(E, cg);
-    for (int c = ln; c < C; c += 32) E.siga[c] = E.sigo[c];
-    __syncwarp();
-    for (int j = 0; j < K; ++j) {
-        for (int c = ln; c < C; c += 32) E.sig[c] = 0.0;
         __syncwarp();
-        if (ln == 0 && j >= 0 && j < E.nslip) E.sig[E.sidx[j]] = 1.0;
+        if (t % M == 0) {  // stages t - M + 1 .. t met every pair once (from the second window on)
+            if (!__any_sync(kAll, big) && t >= 2 * M) break;
+            big = false;
+        }
+    }
+}
+
+// does the bilateral solution -G^-1 b leave a cone (k_bilat: Cholesky of G with floored pivots)?
+// The problem's lanes share the factor's rows; the two substitutions are each lane's own.
+template <int C>
+__device__ bool leaves_cone(Env<C> &E, double mu)
+{
+    using D = Dim<C>;
+    constexpr int M = D::M;
+    double *A = E.A;
+    for (int i = E.c; i < M * M; i += D::L) A[i] = E.G[i];
+    __syncwarp();
+    for (int k = 0; k < M; ++k) {
+        double d = A[k * M + k];
+        for (int j = 0; j < k; ++j) d = fma(-A[k * M + j], A[k * M + j], d);
+        if (d < kTiny) d = kTiny;
+        d = sqrt(d);
+        for (int i = k + 1 + E.c; i < M; i += D::L) {
+            double s = A[i * M + k];
+            for (int j = 0; j < k; ++j) s = fma(-A[i * M + j], A[k * M + j], s);
+            A[i * M + k] = s / d;
+        }
         __syncwarp();
-        grad_once<kC>(E, cg);
-        if (j < E.nslip)
-            for (int i = ln; i < E.nslip; i += 32) {
-                const int c = E.sidx[i];
-                E.Bm[i * C + j] = E.sigo[c] - E.siga[c];
-            }
+        if (E.c == 0) A[k * M + k] = d;
         __syncwarp();
     }
-    // (I - B) sigma = a over the slip contacts: Gauss with partial pivoting, lane 0 (k_solvesig)
-    if (ln == 0) {
-        for (int c = 0; c < C; ++c) E.sig[c] = 0.0;
-        const int n = E.nslip;
-        if (n > 0) {
-            for (int i = 0; i < n; ++i) {
-                for (int j = 0; j < n; ++j) E.Aw[i * C + j] = (i == j ? 1.0 : 0.0) - E.Bm[i * C + j];
-                E.rw[i] = E.siga[E.sidx[i]];
-            }
-            for (int k = 0; k < n; ++k) {
-                int piv = k;
-                double big = fabs(E.Aw[k * C + k]);
-                for (int i = k + 1; i < n; ++i) {
-                    const double v = fabs(E.Aw[i * C + k]);
-                    if (v > big) {
-                        big = v;
-                        piv = i;
-                    }
-                }
-                if (piv != k) {
-                    for (int j = 0; j < n; ++j) {
-                        const double t = E.Aw[k * C + j];
-                        E.Aw[k * C + j] = E.Aw[piv * C + j];
-                        E.Aw[piv * C + j] = t;
-                    }
-                    const double t = E.rw[k];
-                    E.rw[k] = E.rw[piv];
-                    E.rw[piv] = t;
-                }
-                const double d = E.Aw[k * C + k];
-                if (d > kTiny || d < -kTiny)
-                    for (int i = k + 1; i < n; ++i) {
-                        const double f = E.Aw[i * C + k] / d;
-                        for (int j = k; j < n; ++j) E.Aw[i * C + j] = E.Aw[i * C + j] - f * E.Aw[k * C + j];
-                        E.rw[i] = E.rw[i] - f * E.rw[k];
-                    }
-            }
-            for (int ii = 0; ii < n; ++ii) {
-                const int i = n - 1 - ii;
-                double s = E.rw[i];
-                for (int j = i + 1; j < n; ++j) s = s - E.Aw[i * C + j] * E.sig[E.sidx[j]];
-                const double d = E.Aw[i * C + i];
-                if (d > kTiny || d < -kTiny) E.sig[E.sidx[i]] = s / d;
-            }
+    if (E.c == 0) {
+        for (int i = 0; i < M; ++i) {
+            double s = -E.bb[i];
+            for (int j = 0; j < i; ++j) s = fma(-A[i * M + j], E.bw[j], s);
+            E.bw[i] = s / A[i * M + i];
+        }
+        for (int i = M - 1; i >= 0; --i) {
+            double s = E.bw[i];
+            for (int j = i + 1; j < M; ++j) s = fma(-A[j * M + i], E.bw[j], s);
+            E.bw[i] = s / A[i * M + i];
         }
     }
     __syncwarp();
-    grad_once<kC>(E, cg);
+    bool bind = false;
+    if (E.on) {
+        const double *w = E.bw + 3 * E.c;
+        const double lt = sqrt(w[1] * w[1] + w[2] * w[2]);
+        bind = w[0] <= 0.0 || lt > mu * w[0];
+    }
+    const unsigned all = __ballot_sync(kAll, bind);
+    const unsigned mine = (D::L == 32 ? kAll : ((1u << D::L) - 1u)) << (E.g * D::L);
+    __syncwarp();
+    return (all & mine) != 0;
 }
 
-template <int kC>
-__global__ void __launch_bounds__(32, 16) k_admm(b2c_admm P, b2c_admm_params prm)
+// b, G and the column jdir of M^-1 J^T of the warp's problems, one problem after the other with
+// the whole warp (NB:974-1000)
+template <int C>
+__device__ void form(Env<C> &E, const b2c_admm &P, int e0, int jdir)
 {
-    extern __shared__ double s_env[];
-    const int e = blockIdx.x;
-    if (e >= P.n_env) return;
-    const int ln = lane_id(), C = P.nc, NV = P.nv, M = 3 * C;
-    Env E = carve(s_env, C, NV);
-    setup(E, P, prm, e);
-    double resm = CUDART_NAN;
-    if (prm.flags & B2C_ADMM_FORWARD) {
-        for (int i = 0; i < prm.n_iter; ++i) {
-            admm_iter<kC>(E, prm.cg_iters);
-            const int k = prm.chunk > 0 ? i % prm.chunk : i;
-            if (prm.refresh_every > 0 && (k + 1) % prm.refresh_every == 0) resm = refresh<kC>(E, prm.tol, prm.desax != 0);
+    using D = Dim<C>;
+    constexpr int M = D::M;
+    const int nv = P.nv, S = odd(nv), ln = E.ln;
+    double *J = E.stage, *MJ = J + (size_t)M * S, *Mi = MJ + (size_t)M * S;
+    for (int q = 0; q < D::PW; ++q) {
+        const int e = min(e0 + q, P.n_env - 1);
+        const double *Jg = P.J + (size_t)e * M * nv, *Mg = P.Minv + (size_t)e * nv * nv, *vg = P.v_free + (size_t)e * nv;
+        double *G = E.G + (q - E.g) * D::GS, *bb = E.bb + (q - E.g) * D::kVec;
+        for (int i = ln; i < M * nv; i += 32) J[(i / nv) * S + i % nv] = Jg[i];
+        for (int i = ln; i < nv * nv; i += 32) Mi[(i / nv) * S + i % nv] = Mg[i];
+        __syncwarp();
+        for (int i = ln; i < M; i += 32) {
+            double s = 0.0;
+            for (int k = 0; k < nv; ++k) s = fma(J[i * S + k], vg[k], s);
+            bb[i] = P.b_in ? P.b_in[(size_t)e * M + i] : s;
         }
+        for (int i = ln; i < M * nv; i += 32) {
+            const int row = i / nv, k = i - row * nv;
+            double s = 0.0;
+            for (int l = 0; l < nv; ++l) s = fma(Mi[k * S + l], J[row * S + l], s);
+            MJ[row * S + k] = s;
+        }
+        __syncwarp();
+        for (int i = ln; i < M * M; i += 32) {
+            const int row = i / M, col = i - row * M;
+            double s = 0.0;
+            for (int k = 0; k < nv; ++k) s = fma(J[row * S + k], MJ[col * S + k], s);
+            G[i] = s;
+        }
+        for (int i = ln; i < M; i += 32) bb[M + i] = MJ[i * S + jdir];
+        __syncwarp();
+    }
+}
+
+// out[e] = base + M^-1 J^T x of the warp's problems (base: v_free, or dt M^-1 e_jdir), x (M a
+// problem) in E.bw
+template <int C>
+__device__ void respond(Env<C> &E, const b2c_admm &P, int e0, double *out, bool free_v, int jdir, double dt)
+{
+    using D = Dim<C>;
+    constexpr int M = D::M;
+    const int nv = P.nv, ln = E.ln;
+    double *y = E.stage;
+    __syncwarp();
+    for (int q = 0; q < D::PW; ++q) {
+        const int e = e0 + q;
+        if (e >= P.n_env) break;
+        const double *Jg = P.J + (size_t)e * M * nv, *Mg = P.Minv + (size_t)e * nv * nv;
+        const double *x = E.bw + (q - E.g) * D::kVec;
+        if (ln < nv) {
+            double s = 0.0;
+            for (int i = 0; i < M; ++i) s = fma(Jg[(size_t)i * nv + ln], x[i], s);
+            y[ln] = s;
+        }
+        __syncwarp();
+        if (ln < nv) {
+            double s = 0.0;
+            for (int l = 0; l < nv; ++l) s = fma(Mg[(size_t)ln * nv + l], y[l], s);
+            out[(size_t)e * nv + ln] = s + (free_v ? P.v_free[(size_t)e * nv + ln] : dt * Mg[(size_t)ln * nv + jdir]);
+        }
+        __syncwarp();
+    }
+}
+
+// the fixed-branch gradient's per-contact quantities (k_active, NB:546-627)
+struct Branch {
+    int lab;          // 0 open, 1 stick, 2 slip
+    double Z[9], D[3], h1, h2;
+    double Ps[9];     // (Z^T (Gd + eta I) Z + diag D)^-1
+};
+
+template <int C>
+__device__ Branch branch_of(Env<C> &E, const double lam[3], const double u[3], double mu, double eta,
+                            double tol_lam, double tol_rel)
+{
+    using D = Dim<C>;
+    Branch b;
+    double lsc = E.on ? fmax(fabs(lam[0]), fmax(fabs(lam[1]), fabs(lam[2]))) : 0.0;
+#pragma unroll
+    for (int o = D::L / 2; o > 0; o >>= 1) lsc = fmax(lsc, __shfl_xor_sync(kAll, lsc, o));
+    lsc = fmax(lsc, 1.0e-30);
+#pragma unroll
+    for (int i = 0; i < 9; ++i) b.Z[i] = 0.0;
+    b.D[0] = b.D[1] = b.D[2] = 0.0;
+    b.h1 = b.h2 = 0.0;
+    const double lt = sqrt(lam[1] * lam[1] + lam[2] * lam[2]);
+    if (!E.on || lam[0] <= tol_lam + tol_rel * lsc) {
+        b.lab = 0;
+        b.D[0] = b.D[1] = b.D[2] = 1.0;
+    } else if (lt >= mu * lam[0] * (1.0 - tol_rel) - tol_lam) {
+        b.lab = 2;
+        double nw = sqrt(u[1] * u[1] + u[2] * u[2]);
+        if (nw < 1.0e-300) nw = 1.0e-300;
+        b.h1 = u[1] / nw;
+        b.h2 = u[2] / nw;
+        b.Z[0] = 1.0;
+        b.Z[3] = -mu * b.h1;
+        b.Z[6] = -mu * b.h2;
+        b.Z[4] = -b.h2;
+        b.Z[7] = b.h1;
+        b.D[1] = nw / fmax(mu * lam[0], 1.0e-300);
+        b.D[2] = 1.0;
     } else {
-        // the impulses and velocities are given (the gradient of an outside solve)
-        for (int i = ln; i < M; i += 32) {
-            E.zv[i] = P.lam[(size_t)e * M + i];
-            E.u[i] = P.u[(size_t)e * M + i];
-        }
-        __syncwarp();
+        b.lab = 1;
+        b.Z[0] = b.Z[4] = b.Z[8] = 1.0;
     }
-    // v+ = v_free + M^-1 J^T lam (NB:1057-1062)
-    matvec<kC>(E, E.zv, E.tmp, false);
-    if (prm.flags & B2C_ADMM_FORWARD) {
-        for (int i = ln; i < M; i += 32) {
-            P.lam[(size_t)e * M + i] = E.zv[i];
-            P.u[(size_t)e * M + i] = E.u[i];
+    double Q[9], T[9], S[9];
+#pragma unroll
+    for (int i = 0; i < 9; ++i)
+        Q[i] = E.on ? E.G[(3 * E.c + i / 3) * D::M + 3 * E.c + i % 3] + ((i % 4) == 0 ? eta : 0.0) : 0.0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            double s = 0.0;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) s = fma(b.Z[3 * k + i], Q[3 * k + j], s);
+            T[3 * i + j] = s;
         }
-        for (int k = ln; k < NV; k += 32) P.v_plus[(size_t)e * NV + k] = E.vf[k] + E.wv[k];
-        if (ln == 0) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            double s = i == j ? b.D[i] : 0.0;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) s = fma(T[3 * i + k], b.Z[3 * k + j], s);
+            S[3 * i + j] = s;
+        }
+    inv3(S, b.Ps);
+    return b;
+}
+
+// the lane's three rows of Z^T (G + eta I) Z (NB:1040-1043 formed once instead of applied thrice)
+template <int C>
+__device__ __forceinline__ void schur_rows(Env<C> &E, const Branch &b, double eta, double (&S)[3][3 * C])
+{
+    using D = Dim<C>;
+    constexpr int M = D::M;
+    if (E.on)
+        for (int i = 0; i < 9; ++i) E.Z[9 * E.c + i] = b.Z[i];
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        double T[3][3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                double s = 0.0;
+                if (E.on)
+#pragma unroll
+                    for (int k = 0; k < 3; ++k)
+                        s = fma(b.Z[3 * k + i],
+                                E.G[(3 * E.c + k) * M + 3 * c + j] + (c == E.c && k == j ? eta : 0.0), s);
+                T[i][j] = s;
+            }
+        const double *Z = E.Z + 9 * c;
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j)
+                S[i][3 * c + j] = fma(T[i][2], Z[6 + j], fma(T[i][1], Z[3 + j], T[i][0] * Z[j]));
+    }
+    __syncwarp();
+}
+
+// y[n] = (G + eta) x[n], G from shared memory (a few times a gradient)
+template <int C, int N>
+__device__ __forceinline__ void g_times(Env<C> &E, double eta, const double (&x)[N][3], double (&y)[N][3])
+{
+    using D = Dim<C>;
+    constexpr int NS = D::PW * D::XS;
+    double *buf = E.xch + (size_t)E.turn * D::R * NS + E.g * D::XS;
+    E.turn ^= 1;
+    if (E.on)
+#pragma unroll
+        for (int n = 0; n < N; ++n)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) buf[n * NS + 3 * E.c + k] = x[n][k];
+    __syncwarp();
+#pragma unroll
+    for (int n = 0; n < N; ++n)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            double s = 0.0;
+            if (E.on)
+                for (int j = 0; j < D::M; ++j) s = fma(E.G[(3 * E.c + k) * D::M + j], buf[n * NS + j], s);
+            y[n][k] = fma(eta, x[n][k], s);
+        }
+}
+
+// Z^T v
+__device__ __forceinline__ void zt3(const Branch &b, const double v[3], double o[3])
+{
+#pragma unroll
+    for (int j = 0; j < 3; ++j) o[j] = fma(b.Z[6 + j], v[2], fma(b.Z[3 + j], v[1], b.Z[j] * v[0]));
+}
+
+// N right-hand sides through the fixed-branch system: dlam = Z y + pinh, and the slip speed's
+// rate sigo = w . ((G + eta) dlam + db)_t on a slip contact (_grad_once, NB:1162-1170)
+template <int C, int N>
+__device__ __forceinline__ void branch_solve(Env<C> &E, const Branch &b, const double (&S)[3][3 * C], double eta,
+                                             const double (&rhs)[N][3], const double (&pinh)[N][3],
+                                             const double (&db)[N][3], int cg, double (&dl)[N][3], double (&sigo)[N])
+{
+    double y[N][3], t[N][3];
+    pcg<C, N>(E, S, b.D, b.Ps, rhs, y, cg, true, true);
+#pragma unroll
+    for (int n = 0; n < N; ++n)
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            dl[n][k] = fma(b.Z[3 * k + 2], y[n][2], fma(b.Z[3 * k + 1], y[n][1], b.Z[3 * k] * y[n][0])) + pinh[n][k];
+    g_times<C, N>(E, eta, dl, t);
+#pragma unroll
+    for (int n = 0; n < N; ++n)
+        sigo[n] = b.lab == 2 ? fma(b.h1, t[n][1] + db[n][1], b.h2 * (t[n][2] + db[n][2])) : 0.0;
+}
+
+// (I - B) sigma = a over the n slip contacts: Gauss with partial pivoting, one lane (k_solvesig);
+// W (n x n) and r (n) are overwritten
+__device__ inline void eliminate(double *W, int ld, double *r, double *sig, int n)
+{
+    for (int k = 0; k < n; ++k) {
+        int piv = k;
+        double big = fabs(W[k * ld + k]);
+        for (int i = k + 1; i < n; ++i) {
+            const double v = fabs(W[i * ld + k]);
+            if (v > big) {
+                big = v;
+                piv = i;
+            }
+        }
+        if (piv != k) {
+            for (int j = 0; j < n; ++j) {
+                const double t = W[k * ld + j];
+                W[k * ld + j] = W[piv * ld + j];
+                W[piv * ld + j] = t;
+            }
+            const double t = r[k];
+            r[k] = r[piv];
+            r[piv] = t;
+        }
+        const double d = W[k * ld + k];
+        if (d > kTiny || d < -kTiny)
+            for (int i = k + 1; i < n; ++i) {
+                const double f = W[i * ld + k] / d;
+                for (int j = k; j < n; ++j) W[i * ld + j] = fma(-f, W[k * ld + j], W[i * ld + j]);
+                r[i] = fma(-f, r[k], r[i]);
+            }
+    }
+    for (int i = n - 1; i >= 0; --i) {
+        double s = r[i];
+        for (int j = i + 1; j < n; ++j) s = fma(-W[i * ld + j], sig[j], s);
+        const double d = W[i * ld + i];
+        sig[i] = (d > kTiny || d < -kTiny) ? s / d : 0.0;
+    }
+}
+
+// grad_affine (NB:1172-1186) for N directions (pinh, db): dlam.  n_calls - 2 columns of B at most
+// (the rest are zero, as the reference's loop leaves them).
+template <int C, int N>
+__device__ void grad_affine(Env<C> &E, const Branch &b, const double (&S)[3][3 * C], double mu, double eta,
+                            const double (&pinh)[N][3], const double (&db)[N][3], int n_calls, int cg,
+                            double (&dl)[N][3])
+{
+    using D = Dim<C>;
+    double t[N][3], base[N][3], rhs[N][3], so[N];
+    g_times<C, N>(E, eta, pinh, t);
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) t[n][k] = t[n][k] + db[n][k];
+        zt3(b, t[n], base[n]);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) base[n][k] = -base[n][k];
+    }
+    branch_solve<C, N>(E, b, S, eta, base, pinh, db, cg, dl, so);
+    // the rank of this lane's contact among the problem's slip contacts, and their number
+    const unsigned slips = (__ballot_sync(kAll, b.lab == 2) >> (E.g * D::L)) & ((1u << D::L) - 1u);
+    const int rank = __popc(slips & ((1u << E.c) - 1u)), ns = __popc(slips);
+    if (b.lab == 2)
+#pragma unroll
+        for (int n = 0; n < N; ++n) E.a[n * C + rank] = so[n];
+    // B's columns: the response of the slip speeds to a unit sigma
+    int most = ns;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(kAll, most, o));
+    const int K = n_calls - 2;
+    for (int i = E.c; i < C * C; i += D::L) E.Bm[i] = 0.0;
+    __syncwarp();
+    for (int j = 0; j < K && j < most; j += D::R) {
+        double ur[D::R][3], zero[D::R][3], ud[D::R][3], us[D::R];
+#pragma unroll
+        for (int n = 0; n < D::R; ++n)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                zero[n][k] = 0.0;
+                ur[n][k] = k == 0 && b.lab == 2 && rank == j + n ? -mu : 0.0;
+            }
+        branch_solve<C, D::R>(E, b, S, eta, ur, zero, zero, cg, ud, us);
+        if (b.lab == 2)
+#pragma unroll
+            for (int n = 0; n < D::R; ++n)
+                if (j + n < ns && j + n < K) E.Bm[rank * C + j + n] = us[n];
+    }
+    __syncwarp();
+    if (E.c == 0) {
+        double *W = E.A;  // C x C
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+            for (int i = 0; i < ns; ++i)
+                for (int j = 0; j < ns; ++j) W[i * C + j] = (i == j ? 1.0 : 0.0) - E.Bm[i * C + j];
+            eliminate(W, C, E.a + n * C, E.sg + n * C, ns);
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int n = 0; n < N; ++n)
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            rhs[n][k] = k == 0 && b.lab == 2 ? fma(-mu, E.sg[n * C + rank], base[n][k]) : base[n][k];
+    __syncwarp();
+    branch_solve<C, N>(E, b, S, eta, rhs, pinh, db, cg, dl, so);
+}
+
+template <int C>
+__global__ void __launch_bounds__(32, C <= 5 ? 8 : 4) k_admm(b2c_admm P, b2c_admm_params prm)
+{
+    using D = Dim<C>;
+    constexpr int M = D::M;
+    extern __shared__ __align__(16) double s_env[];
+    const int e0 = blockIdx.x * D::PW;
+    Env<C> E = carve<C>(s_env, P.nv);
+    const int e = min(e0 + E.g, P.n_env - 1);
+    const bool live = E.on && e0 + E.g < P.n_env;  // this lane writes its contact's results
+    const bool forward = (prm.flags & B2C_ADMM_FORWARD) != 0;
+    form<C>(E, P, e0, prm.jdir);
+    const double mu = E.on ? P.mu[(size_t)e * C + E.c] : 0.0, icm = 1.0 / (1.0 + mu * mu);
+    double g[3][M], bb[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        bb[k] = E.on ? E.bb[3 * E.c + k] : 0.0;
+#pragma unroll
+        for (int j = 0; j < M; ++j) g[k][j] = E.on ? E.G[(3 * E.c + k) * M + j] : 0.0;
+    }
+    // the diagonal block's largest eigenvalue, eta, the residual's step (k_gd3, k_eta)
+    double W[9];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) W[i] = E.on ? E.G[(3 * E.c + i / 3) * M + 3 * E.c + i % 3] : 0.0;
+    const double gn = eigmax3(W), eta = prm.alpha_eta * gn, gs = gn + eta;
+    const double rhoc = gs > 0.0 ? 1.0 / gs : 1.0;
+    double x[1][3] = {{0.0, 0.0, 0.0}}, zv[1][3] = {{0.0, 0.0, 0.0}}, gam[3] = {0.0, 0.0, 0.0}, u[3] = {0.0, 0.0, 0.0};
+    if (forward) {
+        // rho (k_rho): sqrt(lmin+ lmax) | lmin+ | lmax | the regime's choice | given
+        double rho;
+        if (prm.rho_mode == B2C_ADMM_RHO_GIVEN) {
+            rho = P.rho[e];
+        } else {
+            for (int i = E.c; i < M * M; i += D::L) E.A[i] = E.G[i];
+            __syncwarp();
+            spectrum<C>(E, prm.jacobi_sweeps);
+            double mx = -1.0e300;
+            for (int i = 0; i < M; ++i) mx = fmax(mx, E.A[i * M + i]);
+            const double thr = 1e-12 * mx;
+            double mn = mx;
+            for (int i = 0; i < M; ++i) {
+                const double v = E.A[i * M + i];
+                if (v > thr && v < mn) mn = v;
+            }
+            __syncwarp();
+            rho = sqrt(mn * mx);
+            if (prm.rho_mode == B2C_ADMM_RHO_LMIN) rho = mn;
+            if (prm.rho_mode == B2C_ADMM_RHO_LMAX) rho = mx;
+            if (prm.rho_mode == B2C_ADMM_RHO_REGIME) rho = leaves_cone<C>(E, mu) ? mx : mn;
+        }
+        const double irho = 1.0 / rho;
+        // block-Jacobi preconditioner (k_pjac)
+        double Pj[9], d[3];
+        const double sh = eta + rho;
+#pragma unroll
+        for (int i = 0; i < 9; ++i) W[i] = W[i] + ((i % 4) == 0 ? sh : 0.0);
+        inv3(W, Pj);
+        if (!E.on)
+#pragma unroll
+            for (int i = 0; i < 9; ++i) Pj[i] = 0.0;
+        d[0] = d[1] = d[2] = sh;
+        double sl = 0.0, resm = CUDART_NAN;
+        bool run = true;
+        for (int it = 0; it < prm.n_iter; ++it) {
+            // one iteration (NB:1075-1082)
+            double rhs[1][3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const double q = k == 0 ? fma(mu, sl, bb[0]) : bb[k];
+                rhs[0][k] = -fma(-rho, zv[0][k], q + gam[k]);
+            }
+            pcg<C, 1>(E, g, d, Pj, rhs, x, prm.cg_iters, false, run);
+            double v[3], zn[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) v[k] = fma(gam[k], irho, x[0][k]);
+            proj3(v, mu, icm, zn);
+            if (run) {
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    zv[0][k] = zn[k];
+                    gam[k] = fma(rho, x[0][k] - zn[k], gam[k]);
+                }
+            }
+            const int kk = prm.chunk > 0 ? it % prm.chunk : it;
+            if (prm.refresh_every > 0 && (kk + 1) % prm.refresh_every == 0) {
+                // the Cadoux refresh, the natural residual and the mask (NB:1084-1092, 498-543)
+                double y[1][3];
+                rows_times<C, 1>(E, g, zv, y);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) u[k] = fma(eta, zv[0][k], y[0][k]) + bb[k];
+                sl = sqrt(fma(u[1], u[1], u[2] * u[2]));
+                double q[3], pr[3];
+                q[0] = fma(-rhoc, prm.desax ? fma(mu, sl, u[0]) : u[0], zv[0][0]);
+                q[1] = fma(-rhoc, u[1], zv[0][1]);
+                q[2] = fma(-rhoc, u[2], zv[0][2]);
+                proj3(q, mu, icm, pr);
+                double m = fmax(fabs(zv[0][0] - pr[0]), fmax(fabs(zv[0][1] - pr[1]), fabs(zv[0][2] - pr[2])));
+                // NaN-propagating maximum (k_resmax): fmax drops a NaN, so it is carried beside it
+                double bad = (zv[0][0] - pr[0]) + (zv[0][1] - pr[1]) + (zv[0][2] - pr[2]);
+                if (!E.on) m = bad = 0.0;
+                bad = bad != bad ? 1.0 : 0.0;
+#pragma unroll
+                for (int o = D::L / 2; o > 0; o >>= 1) {
+                    m = fmax(m, __shfl_xor_sync(kAll, m, o));
+                    bad = fmax(bad, __shfl_xor_sync(kAll, bad, o));
+                }
+                resm = bad > 0.0 ? CUDART_NAN : m;
+                if (resm < prm.tol) run = false;
+                if (!__any_sync(kAll, run)) break;  // every problem of the warp is frozen: nothing moves any more
+            }
+        }
+        if (E.on) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                E.bw[3 * E.c + k] = zv[0][k];
+                if (live) {
+                    P.lam[(size_t)e * M + 3 * E.c + k] = zv[0][k];
+                    P.u[(size_t)e * M + 3 * E.c + k] = u[k];
+                }
+            }
+        }
+        if (live && E.c == 0) {
             if (P.res) P.res[e] = resm;
-            if (P.mask) P.mask[e] = E.mask;
-            if (P.rho) P.rho[e] = E.rho;
+            if (P.mask) P.mask[e] = run ? 1 : 0;
+            if (P.rho) P.rho[e] = rho;
+        }
+        respond<C>(E, P, e0, P.v_plus, true, 0, 0.0);  // v+ = v_free + M^-1 J^T lam (NB:1057-1062)
+    } else if (E.on) {
+        // the impulses and velocities are given (the gradient of an outside solve)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            zv[0][k] = P.lam[(size_t)e * M + 3 * E.c + k];
+            u[k] = P.u[(size_t)e * M + 3 * E.c + k];
         }
     }
-    if (prm.flags & (B2C_ADMM_GRADIENT | B2C_ADMM_GRAD_GIVEN)) {
-        build_active(E, 1e-10, 1e-6);
-        const int n_calls = prm.n_calls > 0 ? prm.n_calls : C + 2;
-        const int j = prm.jdir;
-        for (int i = ln; i < M; i += 32) {
-            E.pinh[i] = 0.0;
-            E.dbv[i] = (prm.flags & B2C_ADMM_GRAD_GIVEN) ? P.dbv_in[(size_t)e * M + i] : prm.dt * E.MJ[i * NV + j];
-        }
-        __syncwarp();
-        grad_affine<kC>(E, n_calls, prm.grad_cg);
-        for (int i = ln; i < M; i += 32) P.dlam_tau[(size_t)e * M + i] = E.dlam[i];
-        if (!(prm.flags & B2C_ADMM_GRAD_GIVEN)) {
-            matvec<kC>(E, E.dlam, E.tmp, false);
-            for (int k = ln; k < NV; k += 32) P.dv_tau[(size_t)e * NV + k] = prm.dt * E.Mi[k * NV + j] + E.wv[k];
-            // mu at the first slip contact (k_pmu): pinh = -lam_n w_hat there, db = 0
-            for (int i = ln; i < M; i += 32) {
-                E.pinh[i] = 0.0;
-                E.dbv[i] = 0.0;
-            }
-            __syncwarp();
-            if (ln == 0 && E.nslip > 0) {
-                const int cc = E.sidx[0];
-                E.pinh[3 * cc + 1] = -E.zv[3 * cc] * E.what[3 * cc + 1];
-                E.pinh[3 * cc + 2] = -E.zv[3 * cc] * E.what[3 * cc + 2];
-            }
-            __syncwarp();
-            if (prm.do_mu) grad_affine<kC>(E, n_calls, prm.grad_cg);
-            for (int i = ln; i < M; i += 32) P.dlam_mu[(size_t)e * M + i] = prm.do_mu ? E.dlam[i] : 0.0;
-        }
-        for (int c = ln; c < C; c += 32)
-            P.labels[(size_t)e * C + c] = E.slipf[c] > 0.5 ? 2 : (E.Zm[9 * c] == 0.0 ? 0 : 1);
-        if (ln == 0) P.nslip[e] = E.nslip;
+    if (!(prm.flags & (B2C_ADMM_GRADIENT | B2C_ADMM_GRAD_GIVEN))) return;
+    const bool given = (prm.flags & B2C_ADMM_GRAD_GIVEN) != 0;
+    const Branch b = branch_of<C>(E, zv[0], u, mu, eta, 1e-10, 1e-6);
+    schur_rows<C>(E, b, eta, g);  // from here g holds the rows of Z^T (G + eta I) Z
+    const int n_calls = prm.n_calls > 0 ? prm.n_calls : C + 2;
+    const unsigned slips = (__ballot_sync(kAll, b.lab == 2) >> (E.g * D::L)) & ((1u << D::L) - 1u);
+    // the directions: b (given, or dt J M^-1 e_jdir), and mu at the first slip contact (k_pmu)
+    double dbt[3], pm[3] = {0.0, 0.0, 0.0}, lt[3] = {0.0, 0.0, 0.0}, lm[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        dbt[k] = !E.on ? 0.0 : given ? P.dbv_in[(size_t)e * M + 3 * E.c + k] : prm.dt * E.mjc[3 * E.c + k];
+    if (b.lab == 2 && (slips & ((1u << E.c) - 1u)) == 0) {
+        pm[1] = -zv[0][0] * b.h1;
+        pm[2] = -zv[0][0] * b.h2;
     }
+    const int dirs = !given && prm.do_mu ? 2 : 1;
+    int done = 0;
+    if constexpr (D::R == 2) {
+        if (dirs == 2) {
+            double pin[2][3], db[2][3], dl[2][3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                pin[0][k] = db[1][k] = 0.0;
+                db[0][k] = dbt[k];
+                pin[1][k] = pm[k];
+            }
+            grad_affine<C, 2>(E, b, g, mu, eta, pin, db, n_calls, prm.grad_cg, dl);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                lt[k] = dl[0][k];
+                lm[k] = dl[1][k];
+            }
+            done = 2;
+        }
+    }
+#pragma unroll 1
+    for (int n = done; n < dirs; ++n) {
+        double pin[1][3], db[1][3], dl[1][3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            pin[0][k] = n == 0 ? 0.0 : pm[k];
+            db[0][k] = n == 0 ? dbt[k] : 0.0;
+        }
+        grad_affine<C, 1>(E, b, g, mu, eta, pin, db, n_calls, prm.grad_cg, dl);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            if (n == 0) lt[k] = dl[0][k];
+            else lm[k] = dl[0][k];
+        }
+    }
+    if (E.on)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            E.bw[3 * E.c + k] = lt[k];
+            if (live) {
+                P.dlam_tau[(size_t)e * M + 3 * E.c + k] = lt[k];
+                if (!given) P.dlam_mu[(size_t)e * M + 3 * E.c + k] = lm[k];
+            }
+        }
+    if (live) {
+        P.labels[(size_t)e * C + E.c] = b.lab;
+        if (E.c == 0) P.nslip[e] = __popc(slips);
+    }
+    if (!given) respond<C>(E, P, e0, P.dv_tau, false, prm.jdir, prm.dt);
+}
+
+template <int C>
+static void launch(const b2c_admm &a, const b2c_admm_params &p, cudaStream_t st)
+{
+    const size_t smem = smem_bytes<C>(a.nv);
+    static bool set = false;  // above the 48 KB a launch may have by default
+    if (!set) {
+        cudaFuncSetAttribute(k_admm<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+        set = true;
+    }
+    const int per = Dim<C>::PW;
+    k_admm<C><<<(a.n_env + per - 1) / per, 32, smem, st>>>(a, p);
 }
 
 }  // namespace badmm
@@ -771,7 +962,24 @@ __global__ void __launch_bounds__(32, 16) k_admm(b2c_admm P, b2c_admm_params prm
 extern "C" int64_t b2c_admm_smem_bytes(int32_t nc, int32_t nv)
 {
     if (nc < 1 || nc > B2C_ADMM_MAX_CONTACTS || nv < 1 || nv > B2C_ADMM_MAX_DOFS) return -1;
-    return (int64_t)b2c::badmm::env_bytes(nc, nv);
+    using namespace b2c::badmm;
+    size_t n = 0;
+    switch (nc) {
+#define B2C_ADMM_CASE(k)        \
+    case k:                     \
+        n = smem_bytes<k>(nv);  \
+        break;
+        B2C_ADMM_CASE(1)
+        B2C_ADMM_CASE(2)
+        B2C_ADMM_CASE(3)
+        B2C_ADMM_CASE(4)
+        B2C_ADMM_CASE(5)
+        B2C_ADMM_CASE(6)
+        B2C_ADMM_CASE(7)
+        B2C_ADMM_CASE(8)
+#undef B2C_ADMM_CASE
+    }
+    return (int64_t)n;
 }
 
 extern "C" int32_t b2c_admm_solve(const b2c_admm *a, const b2c_admm_params *p, b2c_stream st)
@@ -802,16 +1010,10 @@ extern "C" int32_t b2c_admm_solve(const b2c_admm *a, const b2c_admm_params *p, b
         return B2C_EARG;
     }
     if (a->n_env == 0) return B2C_OK;
-    const size_t smem = badmm::env_bytes(a->nc, a->nv);
-    static bool attr_set[B2C_ADMM_MAX_CONTACTS + 1] = {};
     switch (a->nc) {
-#define B2C_ADMM_CASE(n)                                                                                  \
-    case n:                                                                                               \
-        if (!attr_set[n]) {                                                                               \
-            cudaFuncSetAttribute(badmm::k_admm<n>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024); \
-            attr_set[n] = true;                                                                           \
-        }                                                                                                 \
-        badmm::k_admm<n><<<a->n_env, 32, smem, stream_of(st)>>>(*a, *p);                                 \
+#define B2C_ADMM_CASE(n)                              \
+    case n:                                           \
+        badmm::launch<n>(*a, *p, stream_of(st));      \
         break;
         B2C_ADMM_CASE(1)
         B2C_ADMM_CASE(2)

@@ -649,10 +649,10 @@ B2C_API int32_t b2c_bncp_vjp(const b2c_bncp *p, const double *glam, double *gb, 
  * Batched proximal ADMM with its adjoint: the reference's BatchProxADMMGPU
  * (src/motion_engine/ncp/ncp_batch_gpu.py:918-1313).  n_env independent problems of nc point
  * contacts on nv generalised velocities each (J: 3 nc x nv rows n, t1, t2 per contact), solved
- * matrix-free (G x = J (M^-1 J^T x), with M^-1 J^T x summed in int64 at a per-problem
- * power-of-two scale, NB:326-388) by ADMM with a block-Jacobi preconditioned CG x-step, the
- * exact cone projection and a per-problem convergence mask; then the fixed-branch adjoint by
- * grad_affine (NB:1172-1186).  One warp per problem runs the whole solve in one launch.
+ * on their Delassus matrices G = J M^-1 J^T (the reference applies G matrix-free, NB:326-388) by
+ * ADMM with a block-Jacobi preconditioned CG x-step, the exact cone projection and a per-problem
+ * convergence mask; then the fixed-branch adjoint by grad_affine (NB:1172-1186).  One lane owns
+ * one contact, a warp 4 to 32 problems, and the whole solve is one launch.
  * ------------------------------------------------------------------------------------------- */
 #define B2C_ADMM_MAX_CONTACTS 8
 #define B2C_ADMM_MAX_DOFS 32
@@ -705,7 +705,7 @@ typedef struct b2c_admm_params {
     int32_t do_mu;          /* also the mu direction */
 } b2c_admm_params;
 
-/* dynamic shared memory of one problem (-1 when nc or nv is out of range) */
+/* dynamic shared memory of one warp's problems (-1 when nc or nv is out of range) */
 B2C_API int64_t b2c_admm_smem_bytes(int32_t nc, int32_t nv);
 B2C_API int32_t b2c_admm_solve(const b2c_admm *a, const b2c_admm_params *p, b2c_stream s);
 
