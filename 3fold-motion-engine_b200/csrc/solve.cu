@@ -84,6 +84,7 @@ struct SolveArgs {
     unsigned int *bar_count;  // the grid barrier's arrival counter
     long long timeout_ns;
     const int *island_info;   // the island partition's statistics (B2C_COLOR_ISLANDS) or NULL
+    int choose;               // the cluster and the grid are both launched: the colouring decides
 };
 
 // The island solve ran this substep (its partition has no island above B2C_ISLAND_MAX_PAIRS
@@ -324,6 +325,21 @@ struct GlobalBodies {
     }
 };
 
+// The same through L1, where one SM alone writes the bodies (one CTA, or a thread of its own).
+struct IslandBodies {
+    float *v, *w, *pv, *po;
+    __device__ __forceinline__ f3 get(int b, int k) const
+    {
+        const float *p = k == 0 ? v : k == 1 ? w : k == 2 ? pv : po;
+        return xyz(reinterpret_cast<const float4 *>(p)[b]);
+    }
+    __device__ __forceinline__ void set(int b, int k, f3 x) const
+    {
+        float *p = k == 0 ? v : k == 1 ? w : k == 2 ? pv : po;
+        reinterpret_cast<float4 *>(p)[b] = f4(x, 0.0f);
+    }
+};
+
 // The impulse word of a contact is (jn, jt1, jt2, jp).  A phase can run the velocity chunk and
 // the position chunk of the same pair on two threads (they read and write disjoint state), so the
 // velocity chunk stores only x, y, z and the position chunk only w.
@@ -342,6 +358,25 @@ __device__ __forceinline__ void store_imp_w(float4 *p, float jp) { reinterpret_c
 // whatever the pair's count), so a pair of up to kRowBatch contacts pays two dependent round
 // trips (record, then the bodies' velocities) however many contacts it has.
 // ---------------------------------------------------------------------------------------------
+// a / b for b > 0, and sqrt, as the IEEE operations give them, with zero kept out of their slow
+// paths: the division of a zero and the root of a zero are computed by a subroutine, which every
+// lane of the warp then waits for (on a B200 0 / x takes 250 cycles and sqrt(0) 125, against 45 for
+// either on ordinary numbers), and both are common here -- an open contact's friction limit is
+// zero, a contact that does not move asks for nothing.  Steps of 10 000 boxes in a pile, of 160
+// piles and of the 10 000-box bead lattice: 2 558 -> 2 413, 2 172 -> 2 057 and 648 -> 600 us (grid
+// form); 48 boxes in one CTA 676 -> 626 us together with their velocities through L1.
+__device__ __forceinline__ float div_pos(float a, float b)
+{
+    const bool zero = a == 0.0f;
+    const float q = (zero ? b : a) / b;
+    return zero ? a : q;
+}
+__device__ __forceinline__ float root(float x)
+{
+    const bool zero = x == 0.0f;
+    const float r = sqrtf(zero ? 1.0f : x);
+    return zero ? x : r;
+}
 __device__ __forceinline__ f3 fma3s(float s, f3 a, f3 b) { return f3{fmaf(s, a.x, b.x), fmaf(s, a.y, b.y), fmaf(s, a.z, b.z)}; }
 __device__ __forceinline__ f3 sel3(bool c, f3 a, f3 b) { return f3{c ? a.x : b.x, c ? a.y : b.y, c ? a.z : b.z}; }
 
@@ -523,7 +558,7 @@ __device__ void pair_velocity(const SolveArgs &a, int s, const BA &B, const RowP
             }
             if (meff >= 1e-12f) {
                 float4 im = cur.im;
-                float dj = -vn / meff;
+                float dj = div_pos(-vn, meff);
                 const float nw = fmaxf(0.0f, im.x + dj);
                 dj = nw - im.x;
                 im.x = nw;
@@ -542,13 +577,13 @@ __device__ void pair_velocity(const SolveArgs &a, int s, const BA &B, const RowP
                 vrel = sub3(va, vb);
                 if (meft1 >= 1e-12f && meft2 >= 1e-12f) {
                     const float o1 = im.y, o2 = im.z;
-                    float a1 = o1 - dot3(vrel, t1) / meft1;
-                    float a2 = o2 - dot3(vrel, t2) / meft2;
-                    const float mag = sqrtf(fmaf(a1, a1, a2 * a2));
+                    float a1 = o1 - div_pos(dot3(vrel, t1), meft1);
+                    float a2 = o2 - div_pos(dot3(vrel, t2), meft2);
+                    const float mag = root(fmaf(a1, a1, a2 * a2));
                     const float lim = mu * im.x;
                     if (mag > lim && mag > 1e-12f) {
-                        a1 = a1 * lim / mag;
-                        a2 = a2 * lim / mag;
+                        a1 = div_pos(a1 * lim, mag);
+                        a2 = div_pos(a2 * lim, mag);
                     }
                     im.y = a1;
                     im.z = a2;
@@ -605,7 +640,7 @@ __device__ void pair_position(const SolveArgs &a, int s, const BA &B, const RowP
             const float meff = wa.w;
             if (meff >= 1e-12f) {
                 const float bias = B2C_BETA * fmaxf(wn.w - B2C_SLOP, 0.0f) / a.dt;
-                float dj = (bias - dot3(rel, nrm)) / meff;
+                float dj = div_pos(bias - dot3(rel, nrm), meff);
                 const float nw = fmaxf(0.0f, jp + dj);
                 dj = nw - jp;
                 store_imp_w(&a.rec.contact(kCImp, k0 + j)[s], nw);
@@ -806,10 +841,10 @@ __device__ void pair_velocity_row(const SolveArgs &a, int s, const BA &B, const 
             const float o1 = im.y, o2 = im.z;
             float a1 = o1 - dot3(vrel, t1) * cur.t1.w;
             float a2 = o2 - dot3(vrel, t2) * cur.rb.w;
-            const float mag = sqrtf(fmaf(a1, a1, a2 * a2));
+            const float mag = root(fmaf(a1, a1, a2 * a2));
             const float lim = mu * im.x;
             if (fric && mag > lim && mag > 1e-12f) {
-                const float sc = lim / mag;
+                const float sc = div_pos(lim, mag);
                 a1 = a1 * sc;
                 a2 = a2 * sc;
             }
@@ -912,6 +947,17 @@ __device__ void pair_position_row(const SolveArgs &a, int s, const BA &B, const 
 // ---------------------------------------------------------------------------------------------
 constexpr int kMaxSolveColors = 512;  // the colouring's cap (kMaxColorsCap)
 
+// The automatic form of a scene of kWidePairs bodies or more is decided on the device, by the
+// pairs of a colour: both the 16-CTA cluster and the grid of every SM are launched (the one that
+// is not wanted returns at once, ~2 us), because the colouring is not known when a captured step
+// is launched.  Narrow colours are latency, and the cluster's barrier is the cheaper one (0.25
+// against 1.3 us); a colour that fills the cluster's warps loops on its 16 SMs.  Measured on a
+// B200, cluster / grid in us per step of two substeps (bead lattice: one): 516 pairs a colour (pile
+// of 3 000 boxes) 1 915 / 2 149; 1 500 (bead lattice of 3 000) 540 / 573; 1 767 (20 000 cubes)
+// 1 277 / 1 171; 1 860 (pile of 10 000) 2 470 / 2 413; 2 390 (160 piles, 67 000 boxes) 2 373 /
+// 2 057; 5 000 (bead lattice of 10 000) 739 / 600; 8 680 (100 000 cubes) 3 275 / 1 813.
+constexpr int kWidePairs = 1700;
+
 // The phases of the persistent solve (both forms).  Task layout of a colour of cnt pairs: velocity (or warm) tasks
 // [0, cnt) and position tasks [P0, P0 + cnt) with P0 = cnt rounded up to a warp, in every pass
 // (a pass without the velocity sweep leaves [0, P0) idle).  So no warp mixes the two kinds,
@@ -926,6 +972,7 @@ __device__ __forceinline__ void solve_phases(const SolveArgs &a, const BA &B)
 {
     const int nc = a.hdr->n_colors;
     if (a.hdr->n_pairs == 0 || nc == 0 || islands_took_solve(a)) return;  // uniform over all CTAs
+    if (a.choose && (kKind == kGrid) != (a.hdr->n_pairs >= (long long)kWidePairs * nc)) return;
     __shared__ int s_cstart[kMaxSolveColors], s_ccount[kMaxSolveColors];
     for (int c = threadIdx.x; c < nc && c < kMaxSolveColors; c += blockDim.x) {
         s_cstart[c] = a.cstart[c];
@@ -1002,7 +1049,7 @@ constexpr int kClusterMax = 16;
 
 __global__ void __launch_bounds__(256, 1) k_color_solve_block(SolveArgs a)
 {
-    const GlobalBodies B{a.v, a.w, a.pv, a.po};
+    const IslandBodies B{a.v, a.w, a.pv, a.po};
     if (a.row) solve_phases<kBlock, true, true>(a, B);
     else if (a.fixed_frame) solve_phases<kBlock, false, true>(a, B);
     else solve_phases<kBlock, false, false>(a, B);
@@ -1156,19 +1203,6 @@ __global__ void __launch_bounds__(kSceneThreads, 2) k_color_solve_scenes(SolveAr
 // the velocity range [0, P) is the island that starts at position t of the island-ordered slot
 // list (isl_at[t] > 0); the position range follows at P rounded up to a warp.
 // ---------------------------------------------------------------------------------------------
-struct IslandBodies {
-    float *v, *w, *pv, *po;
-    __device__ __forceinline__ f3 get(int b, int k) const
-    {
-        const float *p = k == 0 ? v : k == 1 ? w : k == 2 ? pv : po;
-        return xyz(reinterpret_cast<const float4 *>(p)[b]);
-    }
-    __device__ __forceinline__ void set(int b, int k, f3 x) const
-    {
-        float *p = k == 0 ? v : k == 1 ? w : k == 2 ? pv : po;
-        reinterpret_cast<float4 *>(p)[b] = f4(x, 0.0f);
-    }
-};
 
 template <bool kRow, bool kFixed>
 __device__ __forceinline__ void island_tasks(const SolveArgs &a, const int *__restrict__ slots,
@@ -1319,6 +1353,7 @@ int color_solve(const b2c_bodies *b, b2c_contacts *kept, b2c_pairs *pr, b2c_head
     a.bar_count = pr->barrier;
     a.timeout_ns = p->barrier_timeout_ns > 0 ? p->barrier_timeout_ns : 1000000000LL;
     a.island_info = nullptr;
+    a.choose = 0;
     const bool islands = (p->flags & B2C_COLOR_ISLANDS) != 0;
     if (islands && !pr->isl_work) {
         set_error("color_solve: B2C_COLOR_ISLANDS needs b2c_pairs.isl_work");
@@ -1375,6 +1410,8 @@ int color_solve(const b2c_bodies *b, b2c_contacts *kept, b2c_pairs *pr, b2c_head
     if (mode < 0) {
         const int cs = std::min(-mode, max_cluster_size(a.row));
         if (cs >= 2) {
+            // a colour has at most n pairs, so below kWidePairs bodies the cluster always runs
+            a.choose = p->solve_blocks == 0 && !scenes && b->n >= kWidePairs && max_coresident_grid_blocks() > cs;
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(cs);
             cfg.blockDim = dim3(a.row ? kClusterThreadsRow : kClusterThreads);
@@ -1394,6 +1431,7 @@ int color_solve(const b2c_bodies *b, b2c_contacts *kept, b2c_pairs *pr, b2c_head
                 return B2C_ECUDA;
             }
             if ((rc = check_launch("color_solve_cluster"))) return rc;
+            if (a.choose) mode = std::min(kSMs, max_coresident_grid_blocks());
         } else {
             mode = std::min((b->n + 255) / 256, max_coresident_grid_blocks());
         }

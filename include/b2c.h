@@ -294,7 +294,8 @@ typedef struct b2c_color_params {
     float mu;                /* friction */
     float t2d;               /* cross-slip damping of the chunk sweep (1 = full) */
     int32_t color_cap;       /* error when the pair graph needs more colours (<= max_colors) */
-    int32_t solve_blocks;    /* persistent solve shape: 0 = pick from the body count; n > 0 = n CTAs
+    int32_t solve_blocks;    /* persistent solve shape: 0 = pick from the body count and, on
+                                the device, the pairs of a colour; n > 0 = n CTAs
                                 with a grid barrier (1 = one CTA, block barriers); -n = a thread-block
                                 cluster of n CTAs with the hardware cluster barrier;
                                 B2C_SOLVE_SCENES = one CTA per scene (b2c_pairs' scene schedule) */
