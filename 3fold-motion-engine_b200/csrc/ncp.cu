@@ -17,7 +17,7 @@
 //             the contact's dynamic bodies is rebuilt from acc at once (k_apply_c, :583-599: a
 //             colour holds each dynamic body at most once, so the thread that owns the contact
 //             owns those bodies for the phase).  All colours of all iterations run in ONE
-//             persistent launch with a barrier between colours (block or cluster);
+//             persistent launch with a barrier between colours (one CTA, a cluster, a grid);
 //   residual  max_c |lambda_c - proj_K(z_c)| of the same map (k_resid, :601-649).
 //
 // Every sum runs in index order with separately rounded operations (the library is built
@@ -34,10 +34,10 @@ namespace ncp {
 
 constexpr double kScale = 1.0e10;
 constexpr int kColorThreads = 1024;
-constexpr int kSweepThreads = 1024;  // 64 groups of 16 lanes: one contact each
-constexpr int kAdjThreads = 512;     // the reverse sweeps: one thread per contact
 constexpr int kClusterMax = 16;
 constexpr int kMaxColors = 1024;  // the reference's _NCOLMAX
+constexpr int kNarrow = 16;           // contacts a colour, on average, below which one CTA runs the sweeps,
+constexpr int kNarrowContacts = 2048; // of at most this many contacts
 
 enum Stat { kNColors = 0, kCacheValid = 1, kCachedC = 2, kCacheHit = 3, kHits = 4, kMisses = 5, kRounds = 6,
             kError = 7 };
@@ -263,8 +263,30 @@ __device__ __forceinline__ void proj(const T z[3], T mu, T out[3])
     }
 }
 
+enum Kind { kBlock = 0, kCluster = 1, kGrid = 2 };
+
+// What a phase costs is its barrier (0.1 us in one CTA, 0.5 in a cluster, 1.3 over every SM), the
+// contact's chain (~1.3 us) and how many contacts a group has to take one after the other, so the
+// form is the smallest launch that has a group for each contact of an average colour.  Measured
+// on a B200 (us per colour phase, float64; one CTA / cluster of 16 / grid of 148): 12 contacts a
+// colour 1.5 / 2.0 / 3.2, 22 2.4 / 2.0 / 3.2, 85 7.3 / 2.2 / 3.3, 300 24 / 2.5 / 3.3, 400 - / 4.3 / 3.4,
+// 5 000 - / 31 / 4.4.  In float32 the cluster has 640 groups and crosses at 500 to 600.
+struct Form {
+    int asked;  // 0 auto: the launched kernels choose by the colouring; else every launch runs
+    int wide;   // contacts a colour, on average, from which the grid runs
+    __device__ __forceinline__ bool here(int kind, int nc, int ncol) const
+    {
+        if (asked != 0) return true;
+        const long long n = nc;
+        const bool narrow = nc <= kNarrowContacts && n < (long long)kNarrow * ncol;
+        return kind == (narrow ? kBlock : ncol > 0 && n >= (long long)wide * ncol ? kGrid : kCluster);
+    }
+};
+
 template <typename T>
 struct SweepArgs {
+    Form form;
+    int smem_bodies;  // one CTA: the bodies whose state it holds in shared memory (0: none)
     int nc;
     const T *Ja, *Jb, *Minv, *vfree, *mu, *bias, *sep, *rho;
     const int *pa, *pb, *order, *cstart, *ccount, *dyn;
@@ -278,7 +300,6 @@ struct SweepArgs {
     Soft soft;
 };
 
-enum Kind { kBlock = 0, kCluster = 1, kGrid = 2 };
 
 // A recorded update, written by the sweeps: the contact's impulse before it [0, 3), the
 // velocities of its bodies a, b [3, 9), [9, 15) (zero where there is no body), the impulse
@@ -287,25 +308,56 @@ enum Kind { kBlock = 0, kCluster = 1, kGrid = 2 };
 // velocities after the update [21, 27), [27, 33).
 constexpr int kTraceWords = 39;
 
-// The barrier between colours.  The grid form (a cooperative launch, every CTA co-resident) is
-// the arrival-counter barrier of b2c_barrier.cuh over a.bar[0] (cleared by the host before the
-// launch); `epoch` counts the grid barriers of this launch.  Its wait is bounded by
-// a.timeout_ns, after which it sets kErrBarrier and every CTA leaves the sweep.
-template <int kKind, typename T>
-__device__ __forceinline__ bool phase_barrier(const SweepArgs<T> &a, unsigned int &epoch)
+// The barrier between colours, split into an arrive and a wait.  The grid form (a cooperative
+// launch, every CTA co-resident) is the arrival-counter barrier of b2c_barrier.cuh over a.bar[0]
+// (cleared by the host before the launch); `epoch` counts the grid barriers of this launch.  Its
+// wait is bounded by a.timeout_ns, after which it sets kErrBarrier and every CTA leaves the sweep.
+template <int kKind, typename A>
+__device__ __forceinline__ void phase_arrive(const A &a, unsigned int &epoch)
+{
+    if (kKind == kCluster) {
+        asm volatile("barrier.cluster.arrive.release;\n" ::: "memory");
+    } else if (kKind == kGrid) {
+        ++epoch;
+        grid_arrive(a.bar);
+    }
+}
+template <int kKind, typename A>
+__device__ __forceinline__ bool phase_wait(const A &a, unsigned int epoch)
 {
     if (kKind == kBlock) {
         __syncthreads();
         return true;
     }
     if (kKind == kCluster) {
-        cg::this_cluster().sync();
+        asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory");
         return true;
     }
-    ++epoch;
-    grid_arrive(a.bar);
     return grid_wait(a.bar, epoch, a.timeout_ns, a.stats + kError, kErrBarrier);
 }
+
+// a / b correctly rounded from y = RN(1 / b), without a division: each correction q + (a - q b) y
+// takes the quotient's error to its square, the first to within an ulp and the second to the
+// rounded quotient (Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990: with y the rounded reciprocal and q within an ulp, RN(q + r y) = RN(a / b)).
+// The caller keeps a and b away from the ends of the exponent range, where the remainder would
+// not be exact.
+__device__ __forceinline__ double quotient(double a, double b, double y)
+{
+    double q = a * y;
+    q = fma(fma(-q, b, a), y, q);
+    return fma(fma(-q, b, a), y, q);
+}
+__device__ __forceinline__ float quotient(float a, float b, float y)
+{
+    float q = a * y;
+    q = fmaf(fmaf(-q, b, a), y, q);
+    return fmaf(fmaf(-q, b, a), y, q);
+}
+__device__ __forceinline__ bool in_range(double x) { return fabs(x) > 1e-140 && fabs(x) < 1e140; }
+__device__ __forceinline__ bool in_range(float x) { return fabsf(x) > 1e-12f && fabsf(x) < 1e12f; }
+// an int64 sum over the fixed-point scale (a whole number: no exponent near the ends)
+__device__ __forceinline__ double unscale(long long s) { return quotient((double)s, kScale, 1.0 / kScale); }
 
 // One contact update of k_sweep (:485-568): u = bias + Ja v_a + Jb v_b (contact_u's sums), the
 // projection of contact_z's argument, then for each dynamic body the swap of the contact's
@@ -313,108 +365,360 @@ __device__ __forceinline__ bool phase_barrier(const SweepArgs<T> &a, unsigned in
 // body's velocity rebuilt from it (k_apply_c, :583-599).  It runs on a group of kGroup = 16
 // lanes, so that one contact's dependent chain is short: lanes 0..5 form the six 6-term sums of
 // u (row i = lane % 3 of side lane / 3); every lane then has u, z and the projection (the same
-// bits in each); lanes 0..11 each own one velocity component k of one side: row k of the
-// Minv J^T products, the accumulator swap and the velocity rebuild (one division each, in
-// parallel).  Every sum runs in the same order as a one-thread update would.
+// bits in each); lanes 0..11 each own one velocity component k of one side: entry k of J^T
+// lambda, row k of Minv times the side's six entries, the accumulator swap and the velocity
+// rebuild.  Every sum runs in the same order as a one-thread update would.
+//
+// What bounds a colour phase is that chain behind the barrier, so only what depends on the
+// other contacts of the sweep is in it -- the bodies' velocities and accumulators, both loaded
+// at once -- and everything else (SweepPre: the indices, the blocks' and Minv's rows, the
+// impulse the contact holds and its rounded contribution, the reciprocal of 1 + mu^2) is loaded
+// before the barrier's wait.  The two square roots do not wait for each other and
+// run as one instruction sequence on alternate lanes; the two divisions by known numbers
+// (1 + mu^2, the fixed-point scale) are multiply-adds (quotient()).  Of the 2.7 us of a phase of a
+// 16-CTA cluster (240 contacts) the barrier and the stores it waits for take 0.9, the chain 1.3 and
+// the fixed words, when they are loaded inside the phase, 0.5.
+//
+// Measured on a B200 against every load behind the barrier, true divisions and one CTA up to
+// 16 384 contacts: us per colour phase of 300 contacts 18.6 -> 2.5 (float32 15.1 -> 2.3), of 5 000
+// 5.9 -> 4.4; 16 sweeps of 1, 4, 24 and 48 stacks of boxes (488, 1 946, 11 668 and 23 250 contacts)
+// 1 598 -> 990, 3 166 -> 1 540, 13 040 -> 2 010 and 4 219 -> 2 670 us.  Staging the blocks in shared
+// memory with cp.async (1.16 -> 1.27 ms for 20 float32 sweeps of 600 bodies) and the bodies' state
+// in the cluster's distributed shared memory (2.70 -> 2.96 us a phase) were both slower.
 constexpr int kGroup = 16;
+constexpr unsigned kWarp = 0xffffffffu;
 
 template <typename T>
-__device__ __forceinline__ T group_get(T x, int src, unsigned mask)
+__device__ __forceinline__ T group_get(T x, int src)
 {
-    return __shfl_sync(mask, x, src, kGroup);
+    return __shfl_sync(kWarp, x, src, kGroup);
+}
+
+// One contact's task: the contact, its bodies, and bits: 1, 2 the body is dynamic, 4 the group
+// has this contact (a group beyond its colour goes along with its warp on the colour's first).
+struct Task {
+    int c, pa, pb, bits;
+};
+
+// The tasks of a CTA's groups, every colour's first round, in shared memory: a contact keeps its
+// group in every sweep, so the three dependent loads that lead to its words (order, bodies,
+// dynamic flags) are paid once a launch and not behind every barrier, whose acquire empties L1.
+// Colours beyond the table, and later rounds of a colour wider than the launch, take the loads.
+constexpr int kTableBytes = 96 * 1024;
+extern __shared__ int4 s_tasks[];
+
+struct TaskTable {
+    const int *pa, *pb, *order, *dyn;
+    const int *start, *count;  // shared copies of the colour offsets and sizes
+    int per, colors;           // groups of the CTA; colours in the table
+
+    __device__ __forceinline__ Task load(int ci, int t) const
+    {
+        const bool on = t < count[ci];
+        Task k;
+        k.c = order[start[ci] + (on ? t : 0)];
+        k.pa = pa[k.c];
+        k.pb = pb[k.c];
+        k.bits = (k.pa >= 0 && dyn[k.pa] ? 1 : 0) | (k.pb >= 0 && dyn[k.pb] ? 2 : 0) | (on ? 4 : 0);
+        return k;
+    }
+    // task t of colour ci, the CTA's group lg; first: of the group's first round
+    __device__ __forceinline__ Task get(int ci, int t, int lg, bool first) const
+    {
+        if (!first || ci >= colors) return load(ci, t);
+        const int4 w = s_tasks[ci * per + lg];
+        return Task{w.x, w.y, w.z, w.w};
+    }
+};
+
+// every thread of the CTA calls it
+template <typename A>
+__device__ __forceinline__ TaskTable task_table(const A &a, int ncol, int *s_start, int *s_count)
+{
+    for (int c = threadIdx.x; c < ncol; c += blockDim.x) {
+        s_start[c] = a.cstart[c];
+        s_count[c] = a.ccount[c];
+    }
+    __syncthreads();
+    TaskTable tt{a.pa, a.pb, a.order, a.dyn, s_start, s_count, (int)blockDim.x / 16, 0};
+    tt.colors = min(ncol, kTableBytes / (16 * tt.per));
+    for (int i = threadIdx.x; i < tt.colors * tt.per; i += blockDim.x) {
+        const int ci = i / tt.per, lg = i - ci * tt.per;
+        const Task k = tt.load(ci, lg * (int)gridDim.x + (int)blockIdx.x);
+        s_tasks[i] = make_int4(k.c, k.pa, k.pb, k.bits);
+    }
+    __syncthreads();
+    return tt;
+}
+
+// what a contact's update needs besides its bodies' velocities and accumulators
+template <typename T>
+struct SweepPre {
+    Task k;
+    bool dyn;          // this lane's component belongs to a dynamic body
+    T Jr[6];           // lanes 0..5: row lane % 3 of side lane / 3
+    T Jc[3], Mr[6];    // lanes 0..11: column k of the side's block, row k of its body's Minv
+    T lo[3], bias, mu, rho, vf, rden;  // bias: lanes 0..2; rden = 1 / (1 + mu^2)
+    long long qold;    // the rounded contribution of `lo` to this lane's component
+};
+
+// row k of Minv (J^T l) on lane (side, k), minv_jt's order: every lane forms its entry of J^T l
+// and reads its side's six
+template <typename T>
+__device__ __forceinline__ T component(const SweepPre<T> &q, const T l3[3], int l)
+{
+    T t = q.Jc[0] * l3[0];
+    t = t + q.Jc[1] * l3[1];
+    t = t + q.Jc[2] * l3[2];
+    const int base = l < 6 ? 0 : 6;
+    T d = q.Mr[0] * group_get(t, base);
+#pragma unroll
+    for (int j = 1; j < 6; ++j) d = d + q.Mr[j] * group_get(t, base + j);
+    return d;
+}
+
+// the loads of a contact's words ...
+template <typename T>
+__device__ __forceinline__ void sweep_load(const SweepArgs<T> &a, const Task &task, int l, SweepPre<T> &q)
+{
+    q.k = task;
+    const int c = task.c;
+    const int side = l / 6, k = l - 6 * side, b = side == 0 ? task.pa : task.pb;
+#pragma unroll
+    for (int j = 0; j < 6; ++j) q.Jr[j] = T(0);
+    if (l < 6) {
+        const T *J = (l < 3 ? a.Ja : a.Jb) + 18 * (size_t)c + 6 * (l % 3);
+#pragma unroll
+        for (int j = 0; j < 6; ++j) q.Jr[j] = J[j];
+    }
+    q.dyn = side < 2 && (task.bits & (side == 0 ? 1 : 2)) != 0;
+    q.vf = T(0);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) q.Jc[j] = T(0);
+#pragma unroll
+    for (int j = 0; j < 6; ++j) q.Mr[j] = T(0);
+    if (q.dyn) {
+        const T *J = (side == 0 ? a.Ja : a.Jb) + 18 * (size_t)c + k, *M = a.Minv + 36 * (size_t)b + 6 * k;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) q.Jc[j] = J[6 * j];
+#pragma unroll
+        for (int j = 0; j < 6; ++j) q.Mr[j] = M[j];
+        q.vf = a.vfree[6 * (size_t)b + k];
+    }
+#pragma unroll
+    for (int j = 0; j < 3; ++j) q.lo[j] = a.lam[3 * (size_t)c + j];
+    q.bias = l < 3 ? a.bias[3 * (size_t)c + l] : T(0);
+    q.mu = a.mu[c];
+    q.rho = a.rho[c];
+}
+// ... and what is computed from them alone, while the other CTAs arrive
+template <typename T>
+__device__ __forceinline__ void sweep_finish(int l, SweepPre<T> &q)
+{
+    q.rden = T(1) / (T(1) + q.mu * q.mu);
+    q.qold = quant(component(q, q.lo, l));
+}
+
+// Body velocities and accumulators: through L2 where other SMs write them; where one CTA runs
+// the whole sweep, ordinary accesses, to the CTA's own shared copy when it fits (State).
+template <int kKind, typename U>
+__device__ __forceinline__ U shared_load(const U *p)
+{
+    return kKind == kBlock ? *p : __ldcg(p);
+}
+template <int kKind, typename U>
+__device__ __forceinline__ void shared_store(U *p, U x)
+{
+    if (kKind == kBlock) *p = x;
+    else __stcg(p, x);
 }
 
 template <typename T>
-__device__ __forceinline__ void sweep_contact_group(const SweepArgs<T> &a, int c, int it, int l, unsigned mask)
+struct State {
+    T *v;
+    long long *acc;
+};
+
+template <typename T, int kKind>
+__device__ __forceinline__ void sweep_contact_group(const SweepArgs<T> &a, const State<T> &S, const SweepPre<T> &q,
+                                                    int it, int l)
 {
-    const int pa = a.pa[c], pb = a.pb[c];
-    const T lo[3] = {a.lam[3 * (size_t)c], a.lam[3 * (size_t)c + 1], a.lam[3 * (size_t)c + 2]};
-    // the six partial sums of u
-    T part = T(0), vs[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
-    if (l < 6) {
-        const int i = l % 3, side = l / 3, b = side == 0 ? pa : pb;
-        if (b >= 0) {
-            for (int j = 0; j < 6; ++j) vs[j] = __ldcg(a.v + 6 * (size_t)b + j);
-            const T *J = (side == 0 ? a.Ja : a.Jb) + 18 * (size_t)c + 6 * i;
-            T sacc = J[0] * vs[0];
-            for (int j = 1; j < 6; ++j) sacc = sacc + J[j] * vs[j];
-            part = sacc;
-        }
+    const int side = l / 6, k = l - 6 * side, pa = q.k.pa, pb = q.k.pb, bk = side == 0 ? pa : pb;
+    // what the other contacts of the sweep have changed: the velocities and the accumulators
+    T vs[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
+    const int bu = l < 3 ? pa : pb;
+    if (l < 6 && bu >= 0) {
+#pragma unroll
+        for (int j = 0; j < 6; ++j) vs[j] = shared_load<kKind>(S.v + 6 * (size_t)bu + j);
     }
-    T u[3];
-    for (int i = 0; i < 3; ++i) {
-        const T sa = group_get(part, i, mask), sb = group_get(part, 3 + i, mask);
-        T ui = a.bias[3 * (size_t)c + i];
-        if (pa >= 0) ui = ui + sa;
-        if (pb >= 0) ui = ui + sb;
-        u[i] = ui;
-    }
+    long long sacc = 0;
+    if (q.dyn) sacc = shared_load<kKind>(S.acc + 6 * (size_t)bk + k);
+    T part = q.Jr[0] * vs[0];
+#pragma unroll
+    for (int j = 1; j < 6; ++j) part = part + q.Jr[j] * vs[j];
+    // lane i < 3: u_i, then every lane the three
+    const T sb = group_get(part, 3 + l % 3);
+    T ui = q.bias;
+    if (pa >= 0) ui = ui + part;
+    if (pb >= 0) ui = ui + sb;
+    const T u[3] = {group_get(ui, 0), group_get(ui, 1), group_get(ui, 2)};
+    // contact_z and proj: the tangential part of z does not depend on the slip speed, so the odd
+    // lanes take |z_t|, the even ones |u_t|
     T z[3], zn[3];
-    contact_z(u, lo, a.mu[c], a.rho[c], a.desaxce, a.soft, a.sep ? a.sep[c] : T(0), z);
-    proj(z, a.mu[c], zn);
+    z[1] = q.lo[1] - q.rho * u[1];
+    z[2] = q.lo[2] - q.rho * u[2];
+    const bool odd = (l & 1) != 0;
+    const T x1 = odd ? z[1] : u[1], x2 = odd ? z[2] : u[2];
+    const T root = rsq(x1 * x1 + x2 * x2), other = __shfl_xor_sync(kWarp, root, 1, kGroup);
+    const T ut = odd ? other : root, zt = odd ? root : other;
+    if (a.soft.on) {
+        const T sep = a.sep ? a.sep[q.k.c] : T(0);
+        T vb = T(0), ms = T(1), isc = T(0);
+        if (sep > T(0)) {
+            vb = sep * (T)a.soft.p[3];
+        } else if (a.soft.use_bias) {
+            const T t = (T)a.soft.p[1] * (T)a.soft.p[0] * sep;
+            vb = t > -(T)a.soft.p[4] ? t : -(T)a.soft.p[4];
+            ms = (T)a.soft.p[1];
+            isc = (T)a.soft.p[2];
+        }
+        T rn = u[0];
+        if (a.desaxce) rn = rn + q.mu * ut;
+        z[0] = (T(1) - isc) * q.lo[0] - q.rho * (ms * rn + vb);
+    } else {
+        T s0 = u[0];
+        if (a.desaxce) s0 = u[0] + q.mu * ut;
+        z[0] = q.lo[0] - q.rho * s0;
+    }
+    if (zt <= q.mu * z[0]) {
+        zn[0] = z[0];
+        zn[1] = z[1];
+        zn[2] = z[2];
+    } else if (q.mu * zt <= -z[0]) {
+        zn[0] = zn[1] = zn[2] = T(0);
+    } else {
+        const T num = z[0] + q.mu * zt, den = T(1) + q.mu * q.mu;
+        const T s = in_range(num) && in_range(den) ? quotient(num, den, q.rden) : num / den;
+        const T f = q.mu * s / zt;
+        zn[0] = s;
+        zn[1] = f * z[1];
+        zn[2] = f * z[2];
+    }
+    const T d = component(q, zn, l);
+    if (!(q.k.bits & 4)) return;
+    const size_t c = (size_t)q.k.c;
+    if (q.dyn) {
+        sacc = sacc + (quant(d) - q.qold);
+        shared_store<kKind>(S.acc + 6 * (size_t)bk + k, sacc);
+        shared_store<kKind>(S.v + 6 * (size_t)bk + k, q.vf + (T)unscale(sacc));
+    }
+    if (l < 3) a.lam[3 * c + l] = l == 0 ? zn[0] : l == 1 ? zn[1] : zn[2];
     if (a.trace) {
         double *t = a.trace + kTraceWords * ((size_t)it * a.nc + c);
         if (l == 0)
-            for (int k = 0; k < 3; ++k) {
-                t[k] = (double)lo[k];
-                t[18 + k] = (double)zn[k] - (double)lo[k];
-                t[33 + k] = (double)z[k];
-                t[36 + k] = (double)u[k];
+            for (int i = 0; i < 3; ++i) {
+                t[i] = (double)q.lo[i];
+                t[18 + i] = (double)zn[i] - (double)q.lo[i];
+                t[33 + i] = (double)z[i];
+                t[36 + i] = (double)u[i];
             }
         if (l == 0 || l == 3)
-            for (int k = 0; k < 6; ++k) t[(l == 0 ? 3 : 9) + k] = (double)vs[k];
-    }
-    if (l == 0) {
-        a.lam[3 * (size_t)c] = zn[0];
-        a.lam[3 * (size_t)c + 1] = zn[1];
-        a.lam[3 * (size_t)c + 2] = zn[2];
-    }
-    if (l < 12) {
-        const int side = l / 6, k = l % 6, b = side == 0 ? pa : pb;
-        if (b >= 0 && a.dyn[b]) {
-            const T *J = (side == 0 ? a.Ja : a.Jb) + 18 * (size_t)c;
-            const T *M = a.Minv + 36 * (size_t)b + 6 * k;
-            // row k of Minv (J^T l), minv_jt's order, for the new and the old impulse
-            T dn = T(0), dold = T(0);
-            for (int j = 0; j < 6; ++j) {
-                T tn = J[j] * zn[0];
-                tn = tn + J[6 + j] * zn[1];
-                tn = tn + J[12 + j] * zn[2];
-                T to = J[j] * lo[0];
-                to = to + J[6 + j] * lo[1];
-                to = to + J[12 + j] * lo[2];
-                if (j == 0) {
-                    dn = M[0] * tn;
-                    dold = M[0] * to;
-                } else {
-                    dn = dn + M[j] * tn;
-                    dold = dold + M[j] * to;
-                }
-            }
-            long long *p = a.acc + 6 * (size_t)b + k;
-            const long long sacc = __ldcg(p) + (quant(dn) - quant(dold));
-            __stcg(p, sacc);
-            __stcg(a.v + 6 * (size_t)b + k, a.vfree[6 * (size_t)b + k] + (T)((double)sacc / kScale));
-        }
+            for (int i = 0; i < 6; ++i) t[(l == 0 ? 3 : 9) + i] = (double)vs[i];
     }
 }
 
+// A group loads its next task's fixed words while it computes the one before it (kAhead), which
+// takes a second SweepPre of registers and so a smaller CTA.  The grid instead has more groups, one
+// for each contact of the widest colours, and loads between its barrier's arrive and wait, which
+// are apart as long as the loads take.
+template <int kKind>
+constexpr bool kAhead = kKind != kGrid;
 template <typename T, int kKind>
-__global__ void __launch_bounds__(kSweepThreads) k_sweeps(SweepArgs<T> a)
+constexpr int sweep_threads()
+{
+    return kAhead<kKind> ? (sizeof(T) == 4 ? 640 : 384) : sizeof(T) == 4 ? 1024 : 640;
+}
+
+template <typename T, int kKind>
+__global__ void __launch_bounds__(sweep_threads<T, kKind>()) k_sweeps(SweepArgs<T> a)
 {
     const int ncol = a.stats[kNColors];
+    if (ncol == 0 || !a.form.here(kKind, a.nc, ncol)) return;  // uniform over the launch
+    __shared__ int s_start[kMaxColors], s_count[kMaxColors];
+    const TaskTable tt = task_table(a, ncol, s_start, s_count);
+    State<T> S{a.v, a.acc};
+    if (kKind == kBlock && a.smem_bodies) {  // behind the task table
+        S.acc = reinterpret_cast<long long *>(s_tasks + tt.colors * tt.per);
+        S.v = reinterpret_cast<T *>(S.acc + 6 * (size_t)a.smem_bodies);
+        for (int i = threadIdx.x; i < 6 * a.smem_bodies; i += blockDim.x) {
+            S.acc[i] = a.acc[i];
+            S.v[i] = a.v[i];
+        }
+        __syncthreads();
+    }
     // Task slot: one group of kGroup lanes per contact; group g = (group in CTA) x CTAs + CTA,
     // so consecutive contacts of a colour land on different CTAs and a colour narrower than
-    // the launch is spread over every SM of it.  A contact keeps its group in every sweep.
-    const int nb = gridDim.x, groups = nb * (blockDim.x / kGroup);
-    const int g = ((int)threadIdx.x / kGroup) * nb + (int)blockIdx.x, l = (int)threadIdx.x % kGroup;
-    const unsigned mask = 0xFFFFu << (((int)threadIdx.x & 31) & ~(kGroup - 1));
+    // the launch is spread over every SM of it.  A contact keeps its group in every sweep (so
+    // its impulse is written and read by the same lanes).
+    const int nb = gridDim.x, groups = nb * tt.per;
+    const int lg = (int)threadIdx.x / kGroup, g = lg * nb + (int)blockIdx.x, l = (int)threadIdx.x % kGroup;
+    const int g0 = (lg & ~1) * nb + (int)blockIdx.x;  // the warp's first group
+    // One loop over the group's tasks, phase after phase.  A task's fixed words are loaded while the
+    // group's task before it is computed, so that their trip to L2 is on no phase's path, and
+    // worked up while the other CTAs arrive at the barrier.  A contact is always its group's own,
+    // so the impulse among them is final, unless the task before is the same contact (one colour).
+    SweepPre<T> pre = {}, next = {};
     unsigned int epoch = 0;
-    for (int it = 0; it < a.iters; ++it)
-        for (int ci = 0; ci < ncol; ++ci) {
-            const int s0 = a.cstart[ci], cnt = a.ccount[ci];
-            for (int t = g; t < cnt; t += groups) sweep_contact_group(a, a.order[s0 + t], it, l, mask);
-            if (!phase_barrier<kKind>(a, epoch)) return;
+    int it = 0, ci = 0, cnt = s_count[0], t = g, t0 = g0;
+    bool have = t0 < cnt;
+    if (have) {
+        sweep_load(a, tt.get(0, t, lg, true), l, pre);
+        sweep_finish(l, pre);
+    }
+    for (;;) {
+        const bool now = have;
+        const int at = it;
+        if (!kAhead<kKind> && now) sweep_contact_group<T, kKind>(a, S, pre, at, l);
+        t += groups;
+        t0 += groups;
+        const bool more = t0 < cnt;
+        if (!more) {
+            t = g;
+            t0 = g0;
+            if (++ci == ncol) {
+                ci = 0;
+                ++it;
+            }
+            cnt = s_count[ci];
+        }
+        have = it < a.iters && t0 < cnt;
+        if (kAhead<kKind>) {
+            if (have) sweep_load(a, tt.get(ci, t, lg, !more), l, next);
+            if (now) sweep_contact_group<T, kKind>(a, S, pre, at, l);
+        }
+        __syncwarp();
+        if (!more) phase_arrive<kKind>(a, epoch);
+        if (have) {
+            if (!kAhead<kKind>) {
+                sweep_load(a, tt.get(ci, t, lg, !more), l, pre);
+            } else {
+                if (next.k.c == pre.k.c) {
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) next.lo[j] = a.lam[3 * (size_t)next.k.c + j];
+                }
+                pre = next;
+            }
+            sweep_finish(l, pre);
+        }
+        if (!more) {
+            if (!phase_wait<kKind>(a, epoch)) return;
+            if (it == a.iters) break;
+        }
+    }
+    if (kKind == kBlock && a.smem_bodies)
+        for (int i = threadIdx.x; i < 6 * a.smem_bodies; i += blockDim.x) {
+            a.acc[i] = S.acc[i];
+            a.v[i] = S.v[i];
         }
 }
 
@@ -440,118 +744,6 @@ __global__ void k_resid(SweepArgs<T> a, T *__restrict__ res, T *__restrict__ uou
     uout[3 * (size_t)c + 2] = u[2];
     // non-negative reals order like their bit patterns
     atomicMax(res_max, (unsigned long long)__double_as_longlong((double)m));
-}
-
-// Colouring behind the cache, one CTA.
-template <typename T>
-__global__ void __launch_bounds__(kColorThreads)
-    k_color(int nc, int nb, const int *__restrict__ pa, const int *__restrict__ pb, const int *__restrict__ feat,
-            const T *__restrict__ Minv, const int *__restrict__ dyn, b2c_ncp_state st, int use_cache, int max_colors)
-{
-    __shared__ int s_flag, s_left;
-    __shared__ int s_cnt[kMaxColors];
-    const int tid = threadIdx.x;
-    int *S = st.stats;
-    T *cm = reinterpret_cast<T *>(st.cache_minv);
-    if (use_cache && S[kCacheValid] == 1 && S[kCachedC] == nc) {
-        if (tid == 0) s_flag = 0;
-        __syncthreads();
-        int mism = 0;
-        for (int c = tid; c < nc; c += kColorThreads)
-            mism |= (pa[c] != st.cache_pa[c]) | (pb[c] != st.cache_pb[c]) | (feat[c] != st.cache_feat[c]);
-        // the translational block (1/m I) and the dynamic flag (k_cache_cmp, :750-765)
-        for (int i = tid; i < nb; i += kColorThreads)
-            mism |= (Minv[36 * (size_t)i] != cm[4 * (size_t)i]) | (Minv[36 * (size_t)i + 7] != cm[4 * (size_t)i + 1]) |
-                    (Minv[36 * (size_t)i + 14] != cm[4 * (size_t)i + 2]) | ((T)dyn[i] != cm[4 * (size_t)i + 3]);
-        if (mism) atomicOr(&s_flag, 1);
-        __syncthreads();
-        if (s_flag == 0) {
-            if (tid == 0) {
-                S[kCacheHit] = 1;
-                S[kHits] += 1;
-            }
-            return;
-        }
-    }
-    for (int c = tid; c < nc; c += kColorThreads) st.col[c] = -1;
-    int r = 0;
-    bool done = nc == 0;
-    for (; !done && r <= nc && r < max_colors; ++r) {
-        for (int i = tid; i < nb; i += kColorThreads) st.claim[i] = ~0ull;
-        __syncthreads();
-        if (tid == 0) s_left = 0;
-        for (int c = tid; c < nc; c += kColorThreads) {
-            if (st.col[c] >= 0) continue;
-            const unsigned long long k = mix64(((unsigned long long)(pa[c] + 1) * (unsigned long long)(nb + 1) +
-                                                (unsigned long long)(pb[c] + 1)) * 1048576ull +
-                                               (unsigned long long)(unsigned)feat[c]);
-            unsigned long long *claim = reinterpret_cast<unsigned long long *>(st.claim);
-            if (pa[c] >= 0 && dyn[pa[c]]) atomicMin(claim + pa[c], k);
-            if (pb[c] >= 0 && dyn[pb[c]]) atomicMin(claim + pb[c], k);
-        }
-        __syncthreads();
-        for (int c = tid; c < nc; c += kColorThreads) {
-            if (st.col[c] >= 0) continue;
-            const unsigned long long k = mix64(((unsigned long long)(pa[c] + 1) * (unsigned long long)(nb + 1) +
-                                                (unsigned long long)(pb[c] + 1)) * 1048576ull +
-                                               (unsigned long long)(unsigned)feat[c]);
-            bool ok = true;
-            if (pa[c] >= 0 && dyn[pa[c]] && st.claim[pa[c]] != k) ok = false;
-            if (pb[c] >= 0 && dyn[pb[c]] && st.claim[pb[c]] != k) ok = false;
-            if (ok) st.col[c] = r;
-            else atomicAdd(&s_left, 1);
-        }
-        __syncthreads();
-        done = s_left == 0;
-        __syncthreads();  // every thread has read s_left before the next round resets it
-    }
-    const int ncol = done ? (nc > 0 ? r : 0) : r;
-    if (!done || ncol > max_colors || ncol > kMaxColors) {
-        if (tid == 0) {
-            S[kError] |= done ? kErrColorOverflow : kErrColorTimeout;
-            S[kNColors] = 0;
-            S[kCacheValid] = 0;
-            S[kRounds] = r;
-        }
-        return;
-    }
-    for (int k = tid; k < ncol; k += kColorThreads) s_cnt[k] = 0;
-    __syncthreads();
-    for (int c = tid; c < nc; c += kColorThreads) atomicAdd(&s_cnt[st.col[c]], 1);
-    __syncthreads();
-    if (tid == 0) {
-        int acc = 0;
-        for (int k = 0; k < ncol; ++k) {
-            st.cstart[k] = acc;
-            st.ccount[k] = s_cnt[k];
-            const int t = s_cnt[k];
-            s_cnt[k] = acc;
-            acc += t;
-        }
-    }
-    __syncthreads();
-    for (int c = tid; c < nc; c += kColorThreads) st.order[atomicAdd(&s_cnt[st.col[c]], 1)] = c;
-    if (use_cache) {
-        for (int c = tid; c < nc; c += kColorThreads) {
-            st.cache_pa[c] = pa[c];
-            st.cache_pb[c] = pb[c];
-            st.cache_feat[c] = feat[c];
-        }
-        for (int i = tid; i < nb; i += kColorThreads) {
-            cm[4 * (size_t)i] = Minv[36 * (size_t)i];
-            cm[4 * (size_t)i + 1] = Minv[36 * (size_t)i + 7];
-            cm[4 * (size_t)i + 2] = Minv[36 * (size_t)i + 14];
-            cm[4 * (size_t)i + 3] = (T)dyn[i];
-        }
-    }
-    if (tid == 0) {
-        S[kNColors] = ncol;
-        S[kRounds] = r;
-        S[kCacheHit] = 0;
-        S[kCacheValid] = use_cache ? 1 : 0;
-        S[kCachedC] = nc;
-        S[kMisses] += 1;
-    }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -611,89 +803,175 @@ int setup(const b2c_ncp_scene *sc, b2c_ncp_state *st, int warm, cudaStream_t s)
     return check_launch("ncp_setup");
 }
 
-// The same colouring over a cooperative grid: every Jones-Plassmann round is three grid phases
-// (reset the claims; claim; win) with the arrival-counter barrier between them, so a round costs
-// a few microseconds however many contacts there are (the one-CTA form walks all of them with
-// 1024 threads, once per round).  Jones-Plassmann is local -- a contact takes colour r when it
-// holds the smallest key at each of its dynamic bodies among the contacts still uncoloured -- so
-// the colours are those of k_color exactly; only the order of the contacts inside a colour
-// (which thread sweeps which contact) differs, and the sweeps do not depend on it.  Scratch words
-// of the barrier buffer: [8], [9] the uncoloured counts of alternate rounds, [10] the cache
-// mismatch flag (all zero at launch).
+// Colouring behind the cache (Jones-Plassmann over the contacts): a contact takes colour r when it
+// holds the smallest key at each of its dynamic bodies among the contacts still uncoloured.  A
+// round is two phases: every uncoloured contact claims its bodies (atomicMin of its key), then
+// each looks whether it holds them all.  A contact that does takes its bodies' claims back at
+// once: whoever still reads one sees a key or a cleared claim, neither his own, and has lost
+// either way; and a claim left standing belongs to a contact that is still uncoloured, so it is
+// a lower bound that the next round's claims complete.  So nothing is cleared between rounds.
+// A thread keeps its contacts' keys and bodies in registers (kColorHold of them; more are read
+// again each round), so a round is the two barriers and one trip to the claims each, and that is
+// what bounds it: ~60 rounds for a stack of boxes, whatever the number of contacts.  Which
+// launch runs it is the price of its barrier against the contacts a thread walks: one CTA up to
+// two contacts a thread, a cluster up to the same, above it every SM.  Measured on a B200 (float64,
+// us; one CTA / cluster / grid; before: one CTA up to 16 384 contacts and a grid with three
+// barriers a round above) -- stacks of 1 946 contacts 112 / 125 / 175 (before 154), 3 912 176 /
+// 136 / 189 (231), 11 668 611 / 151 / 205 (588), 23 250 1 355 / 207 / 220 (476), 61 941 4 270 / 321 /
+// 258 (522); two-colour lattices of 10 000 contacts 36 (104), of 40 000 58 (93).
+constexpr int kColorHold = 4;
 constexpr int kColorGridThreads = 512;
 
-template <typename T>
-__global__ void __launch_bounds__(kColorGridThreads)
-    k_color_grid(int nc, int nb, const int *__restrict__ pa, const int *__restrict__ pb, const int *__restrict__ feat,
-                 const T *__restrict__ Minv, const int *__restrict__ dyn, b2c_ncp_state st, int use_cache,
-                 int max_colors, long long timeout_ns)
+template <int kKind>
+constexpr int color_threads()
 {
-    __shared__ int s_cnt;
-    const int gid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
+    return kKind == kGrid ? kColorGridThreads : kColorThreads;
+}
+
+template <typename T, int kKind>
+__global__ void __launch_bounds__(color_threads<kKind>())
+    k_color(int nc, int nb, const int *__restrict__ pa, const int *__restrict__ pb, const int *__restrict__ feat,
+            const T *__restrict__ Minv, const int *__restrict__ dyn, b2c_ncp_state st, int use_cache, int max_colors,
+            long long timeout_ns)
+{
+    __shared__ int s_raised, s_seen, s_scan[kMaxColors];
+    const int tid = threadIdx.x, gid = blockIdx.x * blockDim.x + tid, nth = gridDim.x * blockDim.x;
     const bool lead = gid == 0;
     int *S = st.stats;
-    unsigned int *bar = st.barrier;
-    unsigned int epoch = 0;
     T *cm = reinterpret_cast<T *>(st.cache_minv);
+    unsigned long long *claim = reinterpret_cast<unsigned long long *>(st.claim);
+    unsigned int epoch = 0;
     auto sync = [&]() -> bool {
+        if (kKind == kBlock) {
+            __syncthreads();
+            return true;
+        }
+        if (kKind == kCluster) {
+            cg::this_cluster().sync();
+            return true;
+        }
         ++epoch;
-        grid_arrive(bar);
-        return grid_wait(bar, epoch, timeout_ns, S + kError, kErrBarrier);
+        grid_arrive(st.barrier);
+        return grid_wait(st.barrier, epoch, timeout_ns, S + kError, kErrBarrier);
     };
-    auto key_of = [&](int c) -> unsigned long long {
-        return mix64(((unsigned long long)(pa[c] + 1) * (unsigned long long)(nb + 1) + (unsigned long long)(pb[c] + 1)) *
-                         1048576ull +
-                     (unsigned long long)(unsigned)feat[c]);
+    // a barrier that tells whether any thread of the launch raised `flag`; ok: the barrier held.
+    // The count of CTAs that raised one only grows; nobody raises again before all have read it,
+    // since a barrier of the next phase lies between.
+    int seen = 0;
+    if (kKind == kCluster) {
+        if (tid == 0) s_raised = 0;
+        cg::this_cluster().sync();
+    }
+    auto any = [&](bool flag, bool &ok) -> bool {
+        const int mine = __syncthreads_or(flag);
+        ok = true;
+        if (kKind == kBlock) return mine != 0;
+        if (kKind == kCluster) {
+            int *raised = cg::this_cluster().map_shared_rank(&s_raised, 0);
+            if (tid == 0 && mine) atomicAdd(raised, 1);
+            cg::this_cluster().sync();
+            if (tid == 0) s_seen = *(volatile int *)raised;
+            __syncthreads();
+        } else {
+            if (tid == 0 && mine) atomicAdd(st.barrier + 8, 1u);
+            ok = sync();
+            if (tid == 0) s_seen = (int)__ldcg(st.barrier + 8);
+            __syncthreads();
+        }
+        const int now = s_seen;
+        const bool r = now != seen;
+        seen = now;
+        return r;
     };
+    bool ok;
     if (use_cache && S[kCacheValid] == 1 && S[kCachedC] == nc) {
-        int mism = 0;
+        bool mism = false;
         for (int c = gid; c < nc; c += nth)
             mism |= (pa[c] != st.cache_pa[c]) | (pb[c] != st.cache_pb[c]) | (feat[c] != st.cache_feat[c]);
+        // the translational block (1/m I) and the dynamic flag (k_cache_cmp, :750-765)
         for (int i = gid; i < nb; i += nth)
             mism |= (Minv[36 * (size_t)i] != cm[4 * (size_t)i]) | (Minv[36 * (size_t)i + 7] != cm[4 * (size_t)i + 1]) |
                     (Minv[36 * (size_t)i + 14] != cm[4 * (size_t)i + 2]) | ((T)dyn[i] != cm[4 * (size_t)i + 3]);
-        if (mism) atomicOr(bar + 10, 1u);
-        if (!sync()) return;
-        if (__ldcg(bar + 10) == 0u) {
+        const bool miss = any(mism, ok);
+        if (!ok) return;
+        if (!miss) {
             if (lead) {
                 S[kCacheHit] = 1;
                 S[kHits] += 1;
             }
+            // no CTA leaves while another may still read the cluster's counter
+            if (kKind == kCluster) cg::this_cluster().sync();
             return;
         }
     }
-    for (int c = gid; c < nc; c += nth) st.col[c] = -1;
-    unsigned long long *claim = reinterpret_cast<unsigned long long *>(st.claim);
+    // a contact's key and its dynamic bodies (-1: none); alive: not coloured yet
+    struct Held {
+        unsigned long long key;
+        int a, b;
+    };
+    auto held = [&](int c) -> Held {
+        Held h;
+        const int A = pa[c], B = pb[c];
+        h.key = mix64(((unsigned long long)(A + 1) * (unsigned long long)(nb + 1) + (unsigned long long)(B + 1)) *
+                          1048576ull +
+                      (unsigned long long)(unsigned)feat[c]);
+        h.a = A >= 0 && dyn[A] ? A : -1;
+        h.b = B >= 0 && dyn[B] ? B : -1;
+        return h;
+    };
+    auto put = [&](const Held &h) {
+        if (h.a >= 0) atomicMin(claim + h.a, h.key);
+        if (h.b >= 0) atomicMin(claim + h.b, h.key);
+    };
+    // does the contact hold its bodies' claims; then it gives them back
+    auto wins = [&](const Held &h) -> bool {
+        const bool w = (h.a < 0 || __ldcg(claim + h.a) == h.key) && (h.b < 0 || __ldcg(claim + h.b) == h.key);
+        if (w) {
+            if (h.a >= 0) __stcg(claim + h.a, ~0ull);
+            if (h.b >= 0) __stcg(claim + h.b, ~0ull);
+        }
+        return w;
+    };
+    Held mine[kColorHold];
+    unsigned alive = 0;
+#pragma unroll
+    for (int q = 0; q < kColorHold; ++q) {
+        const int c = gid + q * nth;
+        if (c < nc) {
+            mine[q] = held(c);
+            alive |= 1u << q;
+        }
+    }
+    for (int c = gid + kColorHold * nth; c < nc; c += nth) st.col[c] = -1;
+    for (int i = gid; i < nb; i += nth) claim[i] = ~0ull;
+    if (!sync()) return;
     int r = 0;
     bool done = nc == 0;
     for (; !done && r <= nc && r < max_colors; ++r) {
-        for (int i = gid; i < nb; i += nth) claim[i] = ~0ull;
+#pragma unroll
+        for (int q = 0; q < kColorHold; ++q)
+            if (alive >> q & 1) put(mine[q]);
+        for (int c = gid + kColorHold * nth; c < nc; c += nth)
+            if (st.col[c] < 0) put(held(c));
         if (!sync()) return;
-        if (lead) bar[8 + ((r + 1) & 1)] = 0u;  // every CTA has read the previous round's count
-        for (int c = gid; c < nc; c += nth) {
-            if (st.col[c] >= 0) continue;
-            const unsigned long long k = key_of(c);
-            if (pa[c] >= 0 && dyn[pa[c]]) atomicMin(claim + pa[c], k);
-            if (pb[c] >= 0 && dyn[pb[c]]) atomicMin(claim + pb[c], k);
-        }
-        if (!sync()) return;
-        if (threadIdx.x == 0) s_cnt = 0;
-        __syncthreads();
-        int left = 0;
-        for (int c = gid; c < nc; c += nth) {
-            if (st.col[c] >= 0) continue;
-            const unsigned long long k = key_of(c);
-            bool ok = true;
-            if (pa[c] >= 0 && dyn[pa[c]] && __ldcg(claim + pa[c]) != k) ok = false;
-            if (pb[c] >= 0 && dyn[pb[c]] && __ldcg(claim + pb[c]) != k) ok = false;
-            if (ok) st.col[c] = r;
-            else ++left;
-        }
-        if (left) atomicAdd(&s_cnt, left);
-        __syncthreads();
-        if (threadIdx.x == 0 && s_cnt) atomicAdd(bar + 8 + (r & 1), (unsigned)s_cnt);
-        if (!sync()) return;
-        done = __ldcg(bar + 8 + (r & 1)) == 0u;
+        bool left = false;
+#pragma unroll
+        for (int q = 0; q < kColorHold; ++q)
+            if (alive >> q & 1) {
+                if (wins(mine[q])) {
+                    st.col[gid + q * nth] = r;
+                    alive &= ~(1u << q);
+                } else {
+                    left = true;
+                }
+            }
+        for (int c = gid + kColorHold * nth; c < nc; c += nth)
+            if (st.col[c] < 0) {
+                if (wins(held(c))) st.col[c] = r;
+                else left = true;
+            }
+        done = !any(left, ok);
+        if (!ok) return;
     }
     const int ncol = done ? (nc > 0 ? r : 0) : r;
     if (!done || ncol > max_colors || ncol > kMaxColors) {
@@ -703,19 +981,29 @@ __global__ void __launch_bounds__(kColorGridThreads)
             S[kCacheValid] = 0;
             S[kRounds] = r;
         }
+        if (kKind == kCluster) cg::this_cluster().sync();
         return;
     }
-    // counts per colour, then their exclusive scan (one thread), then the scatter with the
-    // counts as cursors (they end where they started)
+    // counts per colour, their exclusive scan (the first CTA), then the scatter with the counts as
+    // cursors (they end where they started)
     for (int k = gid; k < ncol; k += nth) st.ccount[k] = 0;
     if (!sync()) return;
     for (int c = gid; c < nc; c += nth) atomicAdd(st.ccount + st.col[c], 1);
     if (!sync()) return;
-    if (lead) {
-        int acc = 0;
-        for (int k = 0; k < ncol; ++k) {
-            st.cstart[k] = acc;
-            acc += __ldcg(st.ccount + k);
+    if (blockIdx.x == 0) {
+        for (int k = tid; k < ncol; k += blockDim.x) s_scan[k] = __ldcg(st.ccount + k);
+        __syncthreads();
+        if (tid == 0) {
+            int acc = 0;
+            for (int k = 0; k < ncol; ++k) {
+                const int n = s_scan[k];
+                s_scan[k] = acc;
+                acc += n;
+            }
+        }
+        __syncthreads();
+        for (int k = tid; k < ncol; k += blockDim.x) {
+            st.cstart[k] = s_scan[k];
             st.ccount[k] = 0;
         }
     }
@@ -747,82 +1035,158 @@ __global__ void __launch_bounds__(kColorGridThreads)
     }
 }
 
+constexpr size_t kStateBytes = 96 * 1024;  // the body state a single sweep CTA holds: 1000 bodies in float64
+
+bool allow_smem(const void *fn, size_t bytes)
+{
+    const bool ok = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
+    if (!ok) cudaGetLastError();
+    return ok;
+}
+
+// the largest power-of-two cluster (at most kClusterMax) of a kernel that the device holds at once
+int cluster_size_of(const void *fn, int threads, size_t smem)
+{
+    if (smem > 0) allow_smem(fn, smem);
+    cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kClusterMax);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    int cs = 0;
+    if (cudaOccupancyMaxPotentialClusterSize(&cs, fn, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        cs = 1;
+    }
+    int p2 = 1;
+    for (int c = 1; c <= std::min(cs, kClusterMax); c *= 2) p2 = c;
+    return p2;
+}
+
+// CTAs of a kernel the device holds at once (SMs x resident CTAs per SM)
+int grid_blocks_of(const void *fn, int threads, size_t smem)
+{
+    int dev = 0, sms = 0, per = 0;
+    if (smem > 0) allow_smem(fn, smem);
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, threads, smem);
+    return std::min(kBarrierMaxCTAs, std::max(1, sms * per));
+}
+
+// of the sweep kernels, cached per type
+template <typename T>
+int cluster_size()
+{
+    static const int n =
+        cluster_size_of((const void *)k_sweeps<T, kCluster>, sweep_threads<T, kCluster>(), kTableBytes);
+    return n;
+}
+template <typename T>
+int grid_blocks()
+{
+    static const int n = grid_blocks_of((const void *)k_sweeps<T, kGrid>, sweep_threads<T, kGrid>(), kTableBytes);
+    return n;
+}
+
+// one CTA, a cluster or a cooperative grid of a kernel
+int launch_kind(const void *fn, void **args, int kind, int ctas, int threads, size_t smem, const char *what,
+                cudaStream_t s)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    if (kind == kGrid) {
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+    } else {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = ctas;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = kind == kBlock ? 0 : 1;
+    const cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args);
+    if (e != cudaSuccess) {
+        set_error("%s: launch of %d CTAs (%s): %s", what, ctas,
+                  kind == kGrid ? "cooperative" : kind == kCluster ? "cluster" : "one", cudaGetErrorString(e));
+        return B2C_ECUDA;
+    }
+    return check_launch(what);
+}
+
+template <typename A>
+int launch_phases(const void *fn, A &a, int kind, int ctas, int threads, size_t smem, const char *what, cudaStream_t s)
+{
+    if (kind == kGrid) cudaMemsetAsync(a.bar, 0, sizeof(uint32_t), s);  // the arrival count restarts every launch
+    void *args[] = {&a};
+    return launch_kind(fn, args, kind, ctas, threads, smem, what, s);
+}
+
 template <typename T>
 int color(const b2c_ncp_scene *sc, b2c_ncp_state *st, const b2c_ncp_params *p, cudaStream_t s)
 {
     const int maxc = std::min(st->max_colors, kMaxColors);
-    int mode = p->solve_blocks;
-    if (mode == 0) mode = sc->n_c <= 16384 ? 1 : 2;
-    if (mode > 1) {  // a cooperative grid of one CTA per SM (fewer arrivals per barrier)
-        static int nblocks = -1;
-        if (nblocks < 0) {
-            int dev = 0, sms = 0, per = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_color_grid<T>, kColorGridThreads, 0);
-            nblocks = per > 0 ? std::min(kBarrierMaxCTAs, sms) : 1;
-        }
-        if (nblocks > 1) {
-            cudaMemsetAsync(st->barrier, 0, sizeof(uint32_t) * kBarrierWords, s);
-            const long long tmo = p->barrier_timeout_ns > 0 ? p->barrier_timeout_ns : 1000000000LL;
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(nblocks);
-            cfg.blockDim = dim3(kColorGridThreads);
-            cfg.stream = s;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeCooperative;
-            attr[0].val.cooperative = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            const cudaError_t e = cudaLaunchKernelEx(&cfg, k_color_grid<T>, sc->n_c, sc->n_b, sc->pa, sc->pb,
-                                                     sc->feature, (const T *)sc->Minv, st->dyn, *st, p->color_cache,
-                                                     maxc, tmo);
-            if (e != cudaSuccess) {
-                set_error("ncp_color: cooperative launch of %d CTAs: %s", nblocks, cudaGetErrorString(e));
-                return B2C_ECUDA;
-            }
-            return check_launch("ncp_color_grid");
-        }
-    }
-    k_color<T><<<1, kColorThreads, 0, s>>>(sc->n_c, sc->n_b, sc->pa, sc->pb, sc->feature, (const T *)sc->Minv, st->dyn,
-                                           *st, p->color_cache, maxc);
-    return check_launch("ncp_color");
+    static const int clusters = cluster_size_of((const void *)k_color<T, kCluster>, kColorThreads, 0);
+    static const int grid = std::min(kSMs, grid_blocks_of((const void *)k_color<T, kGrid>, kColorGridThreads, 0));
+    int kind = p->solve_blocks > 1 ? kGrid : p->solve_blocks == 1 ? kBlock : kCluster;
+    if (p->solve_blocks == 0)
+        kind = sc->n_c <= 2 * kColorThreads ? kBlock : sc->n_c <= 2 * clusters * kColorThreads ? kCluster : kGrid;
+    if (kind == kCluster && clusters < 2) kind = kGrid;
+    if (kind == kGrid && grid < 2) kind = kBlock;
+    const int ctas = kind == kGrid ? grid : kind == kCluster ? clusters : 1;
+    const void *fn = kind == kGrid ? (const void *)k_color<T, kGrid>
+                     : kind == kCluster ? (const void *)k_color<T, kCluster> : (const void *)k_color<T, kBlock>;
+    if (kind == kGrid) cudaMemsetAsync(st->barrier, 0, sizeof(uint32_t) * kBarrierWords, s);
+    int nc = sc->n_c, nb = sc->n_b, cache = p->color_cache, mc = maxc;
+    const T *Minv = (const T *)sc->Minv;
+    long long tmo = p->barrier_timeout_ns > 0 ? p->barrier_timeout_ns : 1000000000LL;
+    b2c_ncp_state state = *st;
+    void *args[] = {&nc, &nb, (void *)&sc->pa, (void *)&sc->pb, (void *)&sc->feature, &Minv, &st->dyn, &state, &cache,
+                    &mc, &tmo};
+    return launch_kind(fn, args, kind, ctas, kind == kGrid ? kColorGridThreads : kColorThreads, 0, "ncp_color", s);
 }
 
-template <typename T>
-int cluster_size()
-{
-    static int cached = -1;
-    if (cached < 0) {
-        cudaFuncSetAttribute(k_sweeps<T, kCluster>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(kClusterMax);
-        cfg.blockDim = dim3(kSweepThreads);
-        int cs = 0;
-        if (cudaOccupancyMaxPotentialClusterSize(&cs, k_sweeps<T, kCluster>, &cfg) != cudaSuccess) {
-            cudaGetLastError();
-            cs = 1;
-        }
-        int p2 = 1;
-        for (int c = 1; c <= std::min(cs, kClusterMax); c *= 2) p2 = c;
-        cached = p2;
-    }
-    return cached;
-}
+// A phase kernel: its three forms (one CTA, a cluster, a cooperative grid), their threads, and the
+// most CTAs of the cluster and the grid that the device holds at once
+struct PhaseKernel {
+    const void *fn[3];
+    int threads[3];
+    int cluster_max, grid_max;
+};
 
-// CTAs of the grid sweep the device holds at once (SMs x resident CTAs per SM); cached per type
-template <typename T>
-int grid_blocks()
+// Runs a phase kernel in the form asked for (b2c_ncp_params.solve_blocks: 1 one CTA, n > 1 a
+// cooperative grid, -n a cluster) or, for 0, in the one that suits the scene.  block_extra: shared
+// memory of the one CTA behind its task table.
+template <typename A>
+int run_phases(A &a, int asked, const PhaseKernel &k, size_t block_extra, const char *what, cudaStream_t s)
 {
-    static int cached = -1;
-    if (cached < 0) {
-        int dev = 0, sms = 0, per = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sweeps<T, kGrid>, kSweepThreads, 0);
-        cached = std::min(kBarrierMaxCTAs, std::max(1, sms * per));
+    const int nc = a.nc;
+    a.form.asked = asked;
+    a.form.wide = k.cluster_max * (k.threads[kCluster] / kGroup);
+    auto launch = [&](int kind, int ctas) {
+        return launch_phases(k.fn[kind], a, kind, ctas, k.threads[kind],
+                             kTableBytes + (kind == kBlock ? block_extra : 0), what, s);
+    };
+    if (asked > 1 && std::min(asked, k.grid_max) > 1) return launch(kGrid, std::min(asked, k.grid_max));
+    if (asked < 0 && std::min(-asked, k.cluster_max) >= 2) return launch(kCluster, std::min(-asked, k.cluster_max));
+    if (asked != 0 || k.cluster_max < 2) {  // one CTA, asked for or all there is; without clusters the grid
+        const bool grid = asked == 0 && k.grid_max > 1 && nc > kNarrowContacts;
+        a.form.asked = grid ? k.grid_max : 1;
+        return grid ? launch(kGrid, k.grid_max) : launch(kBlock, 1);
     }
-    return cached;
+    // auto: every form that some colouring of nc contacts wants is launched, and the colouring that
+    // the device found lets one of them run (Form::here; the others return at once)
+    if (k.grid_max < 2) a.form.wide = nc + 1;
+    int rc = B2C_OK;
+    if (nc <= kNarrowContacts) rc = launch(kBlock, 1);
+    if (rc == B2C_OK && nc >= kNarrow) rc = launch(kCluster, k.cluster_max);
+    if (rc == B2C_OK && nc >= a.form.wide) rc = launch(kGrid, k.grid_max);
+    return rc;
 }
 
 template <typename T>
@@ -832,57 +1196,14 @@ int sweeps(const b2c_ncp_scene *sc, b2c_ncp_state *st, const b2c_ncp_params *p, 
     if (iters <= 0 || sc->n_c == 0) return B2C_OK;
     SweepArgs<T> a = sweep_args<T>(sc, st, p, iters);
     a.trace = trace;
-    int mode = p->solve_blocks;
-    // auto: one CTA for small scenes; else every SM (the sweep's float64 work needs their issue
-    // rate: on the 40 000-contact lattice a grid of 148 CTAs takes 4.6 ms for 40 sweeps, a
-    // 16-CTA cluster 6.6 ms)
-    if (mode == 0) mode = sc->n_c <= 16384 ? 1 : grid_blocks<T>();
-    if (mode > 1) {  // a cooperative grid of at most the co-resident CTAs
-        const int nblocks = std::min(mode, grid_blocks<T>());
-        if (nblocks > 1) {
-            cudaMemsetAsync(st->barrier, 0, sizeof(uint32_t), s);  // the arrival count restarts every launch
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(nblocks);
-            cfg.blockDim = dim3(kSweepThreads);
-            cfg.stream = s;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeCooperative;
-            attr[0].val.cooperative = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            const cudaError_t e = cudaLaunchKernelEx(&cfg, k_sweeps<T, kGrid>, a);
-            if (e != cudaSuccess) {
-                set_error("ncp_sweeps: cooperative launch of %d CTAs: %s", nblocks, cudaGetErrorString(e));
-                return B2C_ECUDA;
-            }
-            return check_launch("ncp_sweeps_grid");
-        }
-        mode = 1;
-    }
-    if (mode < 0) {
-        const int cs = std::min(-mode, cluster_size<T>());
-        if (cs >= 2) {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(cs);
-            cfg.blockDim = dim3(kSweepThreads);
-            cfg.stream = s;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = cs;
-            attr[0].val.clusterDim.y = 1;
-            attr[0].val.clusterDim.z = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            const cudaError_t e = cudaLaunchKernelEx(&cfg, k_sweeps<T, kCluster>, a);
-            if (e != cudaSuccess) {
-                set_error("ncp_sweeps: cluster launch of %d CTAs: %s", cs, cudaGetErrorString(e));
-                return B2C_ECUDA;
-            }
-            return check_launch("ncp_sweeps_cluster");
-        }
-    }
-    k_sweeps<T, kBlock><<<1, kSweepThreads, 0, s>>>(a);
-    return check_launch("ncp_sweeps");
+    static const bool allowed = allow_smem((const void *)k_sweeps<T, kBlock>, kTableBytes + kStateBytes);
+    const size_t state = 6 * (sizeof(T) + 8) * (size_t)sc->n_b;
+    a.smem_bodies = allowed && state <= kStateBytes ? sc->n_b : 0;
+    static const PhaseKernel k = {
+        {(const void *)k_sweeps<T, kBlock>, (const void *)k_sweeps<T, kCluster>, (const void *)k_sweeps<T, kGrid>},
+        {sweep_threads<T, kBlock>(), sweep_threads<T, kCluster>(), sweep_threads<T, kGrid>()},
+        cluster_size<T>(), grid_blocks<T>()};
+    return run_phases(a, p->solve_blocks, k, a.smem_bodies ? state : 0, "ncp_sweeps", s);
 }
 
 template <typename T>
@@ -921,6 +1242,7 @@ int residual(const b2c_ncp_scene *sc, b2c_ncp_state *st, const b2c_ncp_params *p
 // adjoint of kinematic and static bodies is not kept (their velocity is prescribed).
 // ---------------------------------------------------------------------------------------------
 struct AdjArgs {
+    Form form;
     int nc, nb, iters, desaxce;
     const double *Ja, *Jb, *Minv, *mu, *rho, *lam, *u;
     double *trace;  // null: every reverse sweep at the final iterate (lam, u); else the recorded sweeps
@@ -1055,67 +1377,137 @@ __device__ void adj_contact(const AdjArgs &a, int c)
 // lanes 0..11 one velocity component k of one side each (its vbar, row k of Minv vbar, its
 // share of J Minv vbar -- summed over the lanes by a fixed butterfly -- and its vbar update),
 // every lane the projection and its adjoint.
-__device__ void adj_contact_group(const AdjArgs &a, int c, int it, int l, unsigned mask)
+//
+// The projection's derivative depends on the record alone, so it is formed, with every other
+// word that the other contacts of the sweep do not change (AdjPre), before the barrier's wait;
+// behind the barrier are the bodies' vbar, two small products, three butterflies and the update.
+// Measured on a B200 with the whole update behind the barrier before: forward and backward over a
+// four-step rollout of 24 stacks of boxes (11 668 contacts) 524 -> 76 ms, of 4 stacks 55 ms.
+struct AdjPre {
+    Task k;
+    int b;                      // this lane's body
+    bool mine;                  // lane (side, k) of a dynamic body
+    double *tr;
+    double Jc[3], Mr[6];        // column k of the side's block, row k of Minv
+    double gl[3], mu, rho, s0, u1, u2, q;  // q = -rho mu / |u_t| of the de Saxce term (0 where it has none)
+    double ds[3], df[3], f, zn, z1, z2;    // the projection's derivative: zb = g0 ds + (g_t . z_t) df + f g_t
+    double dsm, dfm, mut;              // and in mu: mub = g0 dsm + (g_t . z_t) dfm + mut zb0
+    double old;                 // the running sum this lane adds to: bias_b (lanes 0..2), mu_b (3), rho_b (4)
+};
+
+__device__ __forceinline__ double *adj_sum(const AdjArgs &a, size_t c, int l)
 {
-    const int A = a.pa[c], B = a.pb[c];
-    const bool dA = A >= 0 && a.dyn[A], dB = B >= 0 && a.dyn[B];
-    double *tr = a.trace + kTraceWords * ((size_t)it * a.nc + c);
-    const double *JA = a.Ja + 18 * (size_t)c, *JB = a.Jb + 18 * (size_t)c;
-    const int side = l / 6, k = l % 6, b = side == 0 ? A : B;
-    const bool mine = l < 12 && (side == 0 ? dA : dB);
-    const double *J = side == 0 ? JA : JB;
-    // only vbar waits on the previous colour; the record and the per-contact sums do not
-    const double w = mine ? __ldcg(a.vb + 6 * (size_t)b + k) : 0.0;
-    const double z[3] = {tr[33], tr[34], tr[35]}, u[3] = {tr[36], tr[37], tr[38]};
-    const double gl0[3] = {a.gl[3 * (size_t)c], a.gl[3 * (size_t)c + 1], a.gl[3 * (size_t)c + 2]};
-    const double mu = a.mu[c], rho = a.rho[c];
-    const double ut = sqrt(u[1] * u[1] + u[2] * u[2]);
-    const double s0 = a.desaxce ? u[0] + mu * ut : u[0];
-    // row k of Minv vbar for this lane's side, then J Minv vbar summed over the lanes
-    double mk = 0.0;
-    {
-        const int base = side * 6;
-        double wj[6];
-        for (int j = 0; j < 6; ++j) wj[j] = group_get(w, (base + j) & (kGroup - 1), mask);
-        if (mine) {
-            const double *M = a.Minv + 36 * (size_t)b + 6 * k;
-            for (int j = 0; j < 6; ++j) mk += M[j] * wj[j];
-        }
+    return l < 3 ? a.bias_b + 3 * c + l : l == 3 ? a.mu_b + c : a.rho_b + c;
+}
+
+// what the contact's own updates change
+__device__ __forceinline__ void adj_own(const AdjArgs &a, int l, AdjPre &q)
+{
+    const size_t c = (size_t)q.k.c;
+#pragma unroll
+    for (int r = 0; r < 3; ++r) q.gl[r] = a.gl[3 * c + r];
+    q.old = l < 5 ? *adj_sum(a, c, l) : 0.0;
+}
+
+__device__ __forceinline__ void adj_load(const AdjArgs &a, const Task &task, int it, int l, AdjPre &q)
+{
+    const int c = task.c;
+    q.k = task;
+    q.tr = a.trace + kTraceWords * ((size_t)it * a.nc + c);
+    const int side = l / 6, k = l - 6 * side;
+    q.b = side == 0 ? task.pa : task.pb;
+    q.mine = side < 2 && (task.bits & (side == 0 ? 1 : 2)) != 0;
+#pragma unroll
+    for (int r = 0; r < 3; ++r) q.Jc[r] = 0.0;
+#pragma unroll
+    for (int j = 0; j < 6; ++j) q.Mr[j] = 0.0;
+    if (q.mine) {
+        const double *J = (side == 0 ? a.Ja : a.Jb) + 18 * (size_t)c + k, *M = a.Minv + 36 * (size_t)q.b + 6 * k;
+#pragma unroll
+        for (int r = 0; r < 3; ++r) q.Jc[r] = J[6 * r];
+#pragma unroll
+        for (int j = 0; j < 6; ++j) q.Mr[j] = M[j];
     }
+    q.zn = q.tr[33];
+    q.z1 = q.tr[34];
+    q.z2 = q.tr[35];
+    q.s0 = q.tr[36];
+    q.u1 = q.tr[37];
+    q.u2 = q.tr[38];
+    q.mu = a.mu[c];
+    q.rho = a.rho[c];
+    adj_own(a, l, q);
+}
+
+__device__ __forceinline__ void adj_finish(const AdjArgs &a, int l, AdjPre &q)
+{
+    const double mu = q.mu, zn = q.zn, z1 = q.z1, z2 = q.z2;
+    // |u_t| on the even lanes, |z_t| on the odd ones
+    const bool odd = (l & 1) != 0;
+    const double x1 = odd ? z1 : q.u1, x2 = odd ? z2 : q.u2;
+    const double root = sqrt(x1 * x1 + x2 * x2), other = __shfl_xor_sync(kWarp, root, 1, kGroup);
+    const double ut = odd ? other : root, zt = odd ? root : other;
+    if (a.desaxce) q.s0 = q.s0 + mu * ut;
+    q.q = a.desaxce && ut > kStickSpeed ? -q.rho * mu / ut : 0.0;
+    q.mut = a.desaxce ? -q.rho * ut : 0.0;
+    // proj's branches (proj_adjoint): inside the cone zb = g, below it 0, else the side's derivative
+    const bool inside = zt <= mu * zn, below = mu * zt <= -zn;
+    q.ds[0] = q.f = inside ? 1.0 : 0.0;
+    q.ds[1] = q.ds[2] = q.df[0] = q.df[1] = q.df[2] = q.dsm = q.dfm = 0.0;
+    if (!inside && !below) {
+        const double den = 1.0 + mu * mu, iden = 1.0 / den, izt = 1.0 / zt;
+        const double sv = (zn + mu * zt) * iden;
+        const double t1 = z1 * izt, t2 = z2 * izt;
+        q.f = mu * sv * izt;
+        q.ds[0] = iden;
+        q.ds[1] = mu * t1 * iden;
+        q.ds[2] = mu * t2 * iden;
+        q.dsm = (zt * den - 2.0 * mu * (zn + mu * zt)) * iden * iden;
+        q.df[0] = mu * iden * izt;
+        q.df[1] = (mu * q.ds[1] - mu * sv * t1 * izt) * izt;
+        q.df[2] = (mu * q.ds[2] - mu * sv * t2 * izt) * izt;
+        q.dfm = (sv + mu * q.dsm) * izt;
+    }
+}
+
+template <int kKind>
+__device__ __forceinline__ void adj_contact_group(const AdjArgs &a, const AdjPre &q, int l)
+{
+    const int side = l / 6, k = l - 6 * side;
+    double *vb = a.vb + 6 * (size_t)(q.mine ? q.b : 0) + k;
+    const double w = q.mine ? shared_load<kKind>(vb) : 0.0;
+    // row k of Minv vbar for this lane's side, then J Minv vbar summed over the lanes
+    const int base = l < 6 ? 0 : 6;
+    double mk = 0.0;
+#pragma unroll
+    for (int j = 0; j < 6; ++j) mk += q.Mr[j] * group_get(w, base + j);
     double jm[3];
+#pragma unroll
     for (int r = 0; r < 3; ++r) {
-        double x = mine ? J[6 * r + k] * mk : 0.0;
-        for (int off = kGroup / 2; off > 0; off >>= 1) x += __shfl_xor_sync(mask, x, off, kGroup);
+        double x = q.Jc[r] * mk;
+#pragma unroll
+        for (int off = kGroup / 2; off > 0; off >>= 1) x += __shfl_xor_sync(kWarp, x, off, kGroup);
         jm[r] = x;
     }
-    double g[3];
-    for (int r = 0; r < 3; ++r) g[r] = gl0[r] + jm[r];
-    double zb[3], mub = 0.0;
-    proj_adjoint(z, mu, g, zb, mub);
-    double ub[3] = {-rho * zb[0], -rho * zb[1], -rho * zb[2]};
-    const double rb = -(zb[0] * s0 + zb[1] * u[1] + zb[2] * u[2]);
-    if (a.desaxce) {
-        mub += -rho * ut * zb[0];
-        if (ut > kStickSpeed) {
-            const double q = -rho * mu / ut;
-            ub[1] += q * u[1] * zb[0];
-            ub[2] += q * u[2] * zb[0];
-        }
-    }
-    if (mine) {
-        __stcg(a.vb + 6 * (size_t)b + k, w + ((J[k] * ub[0] + J[6 + k] * ub[1]) + J[12 + k] * ub[2]));
-        tr[21 + 6 * side + k] = w;
-    } else if (l < 12) {
-        tr[21 + 6 * side + k] = 0.0;
-    }
-    if (l == 0) {
-        for (int r = 0; r < 3; ++r) {
-            a.gl[3 * (size_t)c + r] = zb[r] - jm[r];
-            a.bias_b[3 * (size_t)c + r] += ub[r];
-            tr[15 + r] = ub[r];
-        }
-        a.mu_b[c] += mub;
-        a.rho_b[c] += rb;
+    const double g0 = q.gl[0] + jm[0], g1 = q.gl[1] + jm[1], g2 = q.gl[2] + jm[2];
+    const double gz = g1 * q.z1 + g2 * q.z2;
+    const double zb0 = g0 * q.ds[0] + gz * q.df[0];
+    const double zb1 = g0 * q.ds[1] + q.f * g1 + gz * q.df[1];
+    const double zb2 = g0 * q.ds[2] + q.f * g2 + gz * q.df[2];
+    const double ub0 = -q.rho * zb0, ub1 = -q.rho * zb1 + q.q * q.u1 * zb0, ub2 = -q.rho * zb2 + q.q * q.u2 * zb0;
+    if (!(q.k.bits & 4)) return;
+    if (q.mine) shared_store<kKind>(vb, w + ((q.Jc[0] * ub0 + q.Jc[1] * ub1) + q.Jc[2] * ub2));
+    if (l < 12) q.tr[21 + 6 * side + k] = w;  // zero where the side has no dynamic body
+    const size_t c = (size_t)q.k.c;
+    if (l < 3) {
+        const double ub = l == 0 ? ub0 : l == 1 ? ub1 : ub2;
+        q.tr[15 + l] = ub;
+        a.gl[3 * c + l] = (l == 0 ? zb0 : l == 1 ? zb1 : zb2) - (l == 0 ? jm[0] : l == 1 ? jm[1] : jm[2]);
+        *adj_sum(a, c, l) = q.old + ub;
+    } else if (l == 3) {
+        *adj_sum(a, c, l) = q.old + (g0 * q.dsm + gz * q.dfm + q.mut * zb0);
+    } else if (l == 4) {
+        *adj_sum(a, c, l) = q.old - (zb0 * q.s0 + zb1 * q.u1 + zb2 * q.u2);
     }
 }
 
@@ -1199,6 +1591,7 @@ __device__ void top_projector(const double W[3][3], double lm, double P[3][3])
 // and rho_b through Wbar = -rho^2 rho_b P / k (top_projector).  A group of kGroup lanes per
 // contact: lane (side, k), k < 6, owns column k of its side's block adjoint (3 entries) and of
 // its body's Minv adjoint (6 entries) and walks the sweeps for them.
+template <int kKind>
 __device__ void adj_start_group(const AdjArgs &a, int c, int l, unsigned mask)
 {
     const int A = a.pa[c], B = a.pb[c];
@@ -1224,17 +1617,18 @@ __device__ void adj_start_group(const AdjArgs &a, int c, int l, unsigned mask)
         const double *M = a.Minv + 36 * (size_t)b, *J = (side == 0 ? a.Ja : a.Jb) + 18 * (size_t)c;
         const int vo = side == 0 ? 3 : 9, wo = side == 0 ? 21 : 27;
         double Jc[3] = {0.0, 0.0, 0.0}, Mc[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll 4
         for (int it = 0; it < a.iters; ++it) {
             const double *tr = a.trace + kTraceWords * ((size_t)it * a.nc + c);
             const double ub[3] = {tr[15], tr[16], tr[17]}, vk = tr[vo + k];
-            for (int r = 0; r < 3; ++r) Jc[r] += ub[r] * vk;
-            if (!d) continue;
             const double dl[3] = {tr[18], tr[19], tr[20]};
             double w[6], mk = 0.0;
             for (int j = 0; j < 6; ++j) {
                 w[j] = tr[wo + j];
                 mk += M[6 * k + j] * w[j];
             }
+            for (int r = 0; r < 3; ++r) Jc[r] += ub[r] * vk;
+            if (!d) continue;
             for (int r = 0; r < 3; ++r) Jc[r] += dl[r] * mk;
             const double jt = (J[k] * dl[0] + J[6 + k] * dl[1]) + J[12 + k] * dl[2];
             for (int i = 0; i < 6; ++i) Mc[i] += w[i] * jt;
@@ -1244,7 +1638,7 @@ __device__ void adj_start_group(const AdjArgs &a, int c, int l, unsigned mask)
             // the start: vbar of the sweeps' initial velocities
             double w0[6], m0 = 0.0;
             for (int j = 0; j < 6; ++j) {
-                w0[j] = __ldcg(a.vb + 6 * (size_t)b + j);
+                w0[j] = shared_load<kKind>(a.vb + 6 * (size_t)b + j);
                 m0 += M[6 * k + j] * w0[j];
             }
             const double jt0 = (J[k] * lo[0] + J[6 + k] * lo[1]) + J[12 + k] * lo[2];
@@ -1261,7 +1655,7 @@ __device__ void adj_start_group(const AdjArgs &a, int c, int l, unsigned mask)
             double *Mb = a.Minv_b + 36 * (size_t)b;
             for (int i = 0; i < 6; ++i) {
                 const double jwj = (J[i] * WJ[0][k] + J[6 + i] * WJ[1][k]) + J[12 + i] * WJ[2][k];
-                __stcg(Mb + 6 * i + k, __ldcg(Mb + 6 * i + k) + (Mc[i] + w0[i] * jt0 + jwj));
+                shared_store<kKind>(Mb + 6 * i + k, shared_load<kKind>(Mb + 6 * i + k) + (Mc[i] + w0[i] * jt0 + jwj));
             }
         } else {
             for (int r = 0; r < 3; ++r) Jbar[6 * r + k] += Jc[r];
@@ -1277,23 +1671,21 @@ __device__ void adj_start_group(const AdjArgs &a, int c, int l, unsigned mask)
 template <int kKind>
 __device__ __forceinline__ bool adj_barrier(const AdjArgs &a, unsigned int &epoch)
 {
-    if (kKind == kBlock) {
-        __syncthreads();
-        return true;
-    }
-    if (kKind == kCluster) {
-        cg::this_cluster().sync();
-        return true;
-    }
-    ++epoch;
-    grid_arrive(a.bar);
-    return grid_wait(a.bar, epoch, a.timeout_ns, a.stats + kError, kErrBarrier);
+    phase_arrive<kKind>(a, epoch);
+    return phase_wait<kKind>(a, epoch);
 }
 
 template <int kKind>
-__global__ void __launch_bounds__(kAdjThreads) k_adj_sweeps(AdjArgs a)
+constexpr int adj_threads()
+{
+    return kAhead<kKind> ? 384 : 512;
+}
+
+template <int kKind>
+__global__ void __launch_bounds__(adj_threads<kKind>()) k_adj_sweeps(AdjArgs a)
 {
     const int ncol = a.stats[kNColors];
+    if (!a.form.here(kKind, a.nc, ncol)) return;  // uniform over the launch
     const int nb = gridDim.x, nth = gridDim.x * blockDim.x;
     const int tid = ((((int)threadIdx.x >> 5) * nb + (int)blockIdx.x) << 5) | ((int)threadIdx.x & 31);
     const int gid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1301,18 +1693,55 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_sweeps(AdjArgs a)
     if (a.trace) {
         // the recorded sweeps in reverse (a group of kGroup lanes per contact, the forward's
         // task layout), then their start; vb carries through
-        const int groups = nb * (blockDim.x / kGroup);
-        const int g = ((int)threadIdx.x / kGroup) * nb + (int)blockIdx.x, l = (int)threadIdx.x % kGroup;
+        __shared__ int s_start[kMaxColors], s_count[kMaxColors];
+        const TaskTable tt = task_table(a, ncol, s_start, s_count);
+        const int groups = nb * tt.per;
+        const int lg = (int)threadIdx.x / kGroup, g = lg * nb + (int)blockIdx.x, l = (int)threadIdx.x % kGroup;
+        const int g0 = (lg & ~1) * nb + (int)blockIdx.x;  // the warp's first group
         const unsigned mask = 0xFFFFu << (((int)threadIdx.x & 31) & ~(kGroup - 1));
-        for (int it = a.iters - 1; it >= 0; --it)
-            for (int ci = ncol - 1; ci >= 0; --ci) {
-                const int s0 = a.cstart[ci], cnt = a.ccount[ci];
-                for (int t = g; t < cnt; t += groups) adj_contact_group(a, a.order[s0 + t], it, l, mask);
-                if (!adj_barrier<kKind>(a, epoch)) return;
+        AdjPre pre = {}, next = {};
+        int it = a.iters - 1, ci = ncol - 1, cnt = ncol > 0 ? s_count[ncol - 1] : 0, t = g, t0 = g0;
+        bool have = t0 < cnt;
+        if (have) {
+            adj_load(a, tt.get(ci, t, lg, true), it, l, pre);
+            adj_finish(a, l, pre);
+        }
+        while (it >= 0 && ncol > 0) {
+            const bool now = have;
+            if (!kAhead<kKind> && now) adj_contact_group<kKind>(a, pre, l);
+            t += groups;
+            t0 += groups;
+            const bool more = t0 < cnt;
+            if (!more) {
+                t = g;
+                t0 = g0;
+                if (--ci < 0) {
+                    ci = ncol - 1;
+                    --it;
+                }
+                cnt = s_count[ci];
             }
+            have = it >= 0 && t0 < cnt;
+            if (kAhead<kKind>) {
+                if (have) adj_load(a, tt.get(ci, t, lg, !more), it, l, next);
+                if (now) adj_contact_group<kKind>(a, pre, l);
+            }
+            __syncwarp();
+            if (!more) phase_arrive<kKind>(a, epoch);
+            if (have) {
+                if (!kAhead<kKind>) {
+                    adj_load(a, tt.get(ci, t, lg, !more), it, l, pre);
+                } else {
+                    if (next.k.c == pre.k.c) adj_own(a, l, next);
+                    pre = next;
+                }
+                adj_finish(a, l, pre);
+            }
+            if (!more && !phase_wait<kKind>(a, epoch)) return;
+        }
         for (int ci = 0; ci < ncol; ++ci) {
             const int s0 = a.cstart[ci], cnt = a.ccount[ci];
-            for (int t = g; t < cnt; t += groups) adj_start_group(a, a.order[s0 + t], l, mask);
+            for (int t = g; t < cnt; t += groups) adj_start_group<kKind>(a, a.order[s0 + t], l, mask);
             if (!adj_barrier<kKind>(a, epoch)) return;
         }
         for (int i = gid; i < 6 * a.nb; i += nth) {
@@ -1389,35 +1818,14 @@ int adjoint_sweeps(const b2c_ncp_scene *sc, b2c_ncp_state *st, const b2c_ncp_par
     a.timeout_ns = p->barrier_timeout_ns > 0 ? p->barrier_timeout_ns : 1000000000LL;
     cudaMemsetAsync(vb, 0, sizeof(double) * 6 * (size_t)sc->n_b, s);
     if (trace) cudaMemsetAsync(st->res, 0, sizeof(double) * (size_t)sc->n_c, s);
-    int mode = p->solve_blocks;
-    if (mode == 0) mode = sc->n_c <= 16384 ? 1 : grid_blocks<double>();
-    if (mode > 1) {
-        int per = 0, dev = 0, sms = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_adj_sweeps<kGrid>, kAdjThreads, 0);
-        const int nblocks = std::min(std::min(mode, kBarrierMaxCTAs), std::max(1, sms * per));
-        if (nblocks > 1) {
-            cudaMemsetAsync(st->barrier, 0, sizeof(uint32_t), s);
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(nblocks);
-            cfg.blockDim = dim3(kAdjThreads);
-            cfg.stream = s;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeCooperative;
-            attr[0].val.cooperative = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            const cudaError_t e = cudaLaunchKernelEx(&cfg, k_adj_sweeps<kGrid>, a);
-            if (e != cudaSuccess) {
-                set_error("ncp_adjoint: cooperative launch of %d CTAs: %s", nblocks, cudaGetErrorString(e));
-                return B2C_ECUDA;
-            }
-            return check_launch("ncp_adjoint_grid");
-        }
-    }
-    k_adj_sweeps<kBlock><<<1, kAdjThreads, 0, s>>>(a);
-    return check_launch("ncp_adjoint");
+    static const bool allowed = allow_smem((const void *)k_adj_sweeps<kBlock>, kTableBytes);
+    (void)allowed;
+    static const PhaseKernel k = {
+        {(const void *)k_adj_sweeps<kBlock>, (const void *)k_adj_sweeps<kCluster>, (const void *)k_adj_sweeps<kGrid>},
+        {adj_threads<kBlock>(), adj_threads<kCluster>(), adj_threads<kGrid>()},
+        cluster_size_of((const void *)k_adj_sweeps<kCluster>, adj_threads<kCluster>(), kTableBytes),
+        grid_blocks_of((const void *)k_adj_sweeps<kGrid>, adj_threads<kGrid>(), kTableBytes)};
+    return run_phases(a, p->solve_blocks, k, 0, "ncp_adjoint", s);
 }
 
 }  // namespace ncp
