@@ -8,17 +8,23 @@ namespace b2c {
 struct GridView {
     int dx, dy, dz;
     float inv;  // 1 / cell
+    int pow2;   // every dim is a power of two, as the engines choose them: a wrap is a mask
 };
 
-__device__ __forceinline__ int wrapi(int a, int m)
+// The neighbour search of a bead wraps six coordinates for each of its 9 to 16 columns: as
+// remainders, most of its instructions.  Measured on a
+// B200, the neighbour passes of 10 000 bead boxes (480 000 beads), remainders and a square root a
+// candidate before: contacts of the Jacobi engine 62 -> 54 us, count 46 -> 36, emission 21 -> 18.
+__device__ __forceinline__ int wrapi(int a, int m, int pow2)
 {
+    if (pow2) return a & (m - 1);
     int r = a % m;
     return r < 0 ? r + m : r;
 }
 __device__ __forceinline__ int cellc(float x, float inv) { return (int)floorf(x * inv); }
 __device__ __forceinline__ int bucket_of(const GridView &g, int ix, int iy, int iz)
 {
-    return (wrapi(ix, g.dx) * g.dy + wrapi(iy, g.dy)) * g.dz + wrapi(iz, g.dz);
+    return (wrapi(ix, g.dx, g.pow2) * g.dy + wrapi(iy, g.dy, g.pow2)) * g.dz + wrapi(iz, g.dz, g.pow2);
 }
 
 // Query block of a point: every cell within 2R plus a 1 % margin, so a neighbour at a cell
@@ -39,7 +45,12 @@ __device__ __forceinline__ QueryRange query_range(f3 p, float r, float inv)
     return q;
 }
 
-inline GridView view_of(const b2c_grid *g) { return GridView{g->dim_x, g->dim_y, g->dim_z, 1.0f / g->cell}; }
+inline GridView view_of(const b2c_grid *g)
+{
+    auto pow2 = [](int d) { return (d & (d - 1)) == 0; };
+    return GridView{g->dim_x, g->dim_y, g->dim_z, 1.0f / g->cell,
+                    pow2(g->dim_x) && pow2(g->dim_y) && pow2(g->dim_z) ? 1 : 0};
+}
 // every array of a grid present and its dims at least 8 per axis (the wrap-around query needs it)
 inline bool grid_valid(const b2c_grid *g)
 {
@@ -62,8 +73,11 @@ __device__ __forceinline__ void visit_slots(int i, f3 xi, int bi, const float4 *
         if (j > i && __float_as_int(p.w) != bi) {
             const f3 xj = xyz(p);
             const f3 dvec = sub3(xi, xj);
-            const float dist = len3(dvec);
-            if (dist < B2C_2R && dist > 1e-9f) f(j, xj, dvec, dist);
+            const float d2 = dot3(dvec, dvec);
+            if (d2 < 0.0101f) {  // (2R)^2 = 0.01: farther ones need no square root
+                const float dist = sqrtf(d2);
+                if (dist < B2C_2R && dist > 1e-9f) f(j, xj, dvec, dist);
+            }
         }
     }
 }
