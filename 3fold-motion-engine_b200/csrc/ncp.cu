@@ -269,7 +269,7 @@ enum Kind { kBlock = 0, kCluster = 1, kGrid = 2 };
 // contact's chain (~1.3 us) and how many contacts a group has to take one after the other, so the
 // form is the smallest launch that has a group for each contact of an average colour.  Measured
 // on a B200 (us per colour phase, float64; one CTA / cluster of 16 / grid of 148): 12 contacts a
-// colour 1.5 / 2.0 / 3.2, 22 2.4 / 2.0 / 3.2, 85 7.3 / 2.2 / 3.3, 300 24 / 2.5 / 3.3, 400 - / 4.3 / 3.4,
+// colour 1.5 / 2.0 / 3.2, 22 2.4 / 2.0 / 3.2, 85 7.3 / 2.1 / 3.2, 300 24 / 2.3 / 3.3, 400 - / 4.3 / 3.4,
 // 5 000 - / 31 / 4.4.  In float32 the cluster has 640 groups and crosses at 500 to 600.
 struct Form {
     int asked;  // 0 auto: the launched kernels choose by the colouring; else every launch runs
@@ -316,7 +316,7 @@ template <int kKind, typename A>
 __device__ __forceinline__ void phase_arrive(const A &a, unsigned int &epoch)
 {
     if (kKind == kCluster) {
-        asm volatile("barrier.cluster.arrive.release;\n" ::: "memory");
+        cluster_arrive();
     } else if (kKind == kGrid) {
         ++epoch;
         grid_arrive(a.bar);
@@ -380,10 +380,10 @@ __device__ __forceinline__ double unscale(long long s) { return quotient((double
 // the fixed words, when they are loaded inside the phase, 0.5.
 //
 // Measured on a B200 against every load behind the barrier, true divisions and one CTA up to
-// 16 384 contacts: us per colour phase of 300 contacts 18.6 -> 2.5 (float32 15.1 -> 2.3), of 5 000
+// 16 384 contacts: us per colour phase of 300 contacts 18.6 -> 2.3 (float32 15.1 -> 2.1), of 5 000
 // 5.9 -> 4.4; 16 sweeps of 1, 4, 24 and 48 stacks of boxes (488, 1 946, 11 668 and 23 250 contacts)
-// 1 598 -> 990, 3 166 -> 1 540, 13 040 -> 2 010 and 4 219 -> 2 670 us.  Staging the blocks in shared
-// memory with cp.async (1.16 -> 1.27 ms for 20 float32 sweeps of 600 bodies) and the bodies' state
+// 1 598 -> 990, 3 166 -> 1 530, 13 040 -> 1 945 and 4 219 -> 2 670 us.  Staging the blocks in shared
+// memory with cp.async (1.16 -> 1.27 ms for 60 float32 sweeps of 600 bodies) and the bodies' state
 // in the cluster's distributed shared memory (2.70 -> 2.96 us a phase) were both slower.
 constexpr int kGroup = 16;
 constexpr unsigned kWarp = 0xffffffffu;
@@ -1382,7 +1382,7 @@ __device__ void adj_contact(const AdjArgs &a, int c)
 // word that the other contacts of the sweep do not change (AdjPre), before the barrier's wait;
 // behind the barrier are the bodies' vbar, two small products, three butterflies and the update.
 // Measured on a B200 with the whole update behind the barrier before: forward and backward over a
-// four-step rollout of 24 stacks of boxes (11 668 contacts) 524 -> 76 ms, of 4 stacks 55 ms.
+// four-step rollout of 24 stacks of boxes (11 668 contacts) 524 -> 75 ms, of 4 stacks 55 ms.
 struct AdjPre {
     Task k;
     int b;                      // this lane's body
