@@ -765,9 +765,9 @@ def run_admm(args, wl):
     alg = B * (3 * C * NV + NV * NV + NV + C) * 8 + B * (2 * 3 * C * 3 + NV + 2 * NV) * 8  # inputs once, outputs
     roof = {"bound": "hbm", "achieved": alg / (both_ms / 1e3) / 1e9, "peak": peaks["hbm_gbs"], "unit": "GB/s",
             "frac": alg / (both_ms / 1e3) / 1e9 / peaks["hbm_gbs"], "traffic": None, "peak_kind": peak_kind,
-            "kernel": "k_admm (one warp per problem: set-up, ADMM, active set, grad_affine in shared memory)",
+            "kernel": "k_admm (one lane a contact: set-up, ADMM, active set, grad_affine on the dense Delassus matrix)",
             "launch_ms": both_ms, "algorithmic_bytes_per_launch": alg,
-            "note": "latency-bound: each warp iterates its problem in shared memory; the inputs are read once"}
+            "note": "latency- and FP64-issue-bound: the problems iterate in registers; the inputs are read once"}
     if rank == 0:
         line = {"metric": "env-steps/s", "value": value, "unit": "env-steps/s", "n_gpus": world,
                 "steps": args.steps, "warmup": args.warmup, "ms_per_step": both_ms, "higher_is_better": True,
@@ -881,9 +881,9 @@ def run_adjoint(args, wl):
     alg = B * (n * n + n + n // 3 + n) * 8  # G, b, mu read, lambda written, per launch
     roof = {"bound": "hbm", "achieved": alg / (fwd_ms / 1e3) / 1e9, "peak": peaks["hbm_gbs"], "unit": "GB/s",
             "frac": alg / (fwd_ms / 1e3) / 1e9 / peaks["hbm_gbs"], "traffic": None, "peak_kind": peak_kind,
-            "kernel": "k_bncp_solve (one warp per problem, PGS sweeps to the residual)",
+            "kernel": "k_bncp_solve (one lane a contact, PGS sweeps to the residual)",
             "launch_ms": fwd_ms, "algorithmic_bytes_per_launch": alg,
-            "note": "latency-bound: each warp iterates its problem in shared memory; the bytes are read once"}
+            "note": "latency-bound: the problems iterate in registers and shared memory; the bytes are read once"}
     if rank == 0:
         line = {"metric": "env-steps/s", "value": value, "unit": "env-steps/s", "n_gpus": world,
                 "steps": args.steps, "warmup": args.warmup, "ms_per_step": fwd_ms, "higher_is_better": True,
