@@ -947,11 +947,8 @@ template <int C>
 static void launch(const b2c_admm &a, const b2c_admm_params &p, cudaStream_t st)
 {
     const size_t smem = smem_bytes<C>(a.nv);
-    static bool set = false;  // above the 48 KB a launch may have by default
-    if (!set) {
-        cudaFuncSetAttribute(k_admm<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-        set = true;
-    }
+    // above the 48 KB a launch may have by default; the opt-in is the device's, so for every launch
+    cudaFuncSetAttribute(k_admm<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
     const int per = Dim<C>::PW;
     k_admm<C><<<(a.n_env + per - 1) / per, 32, smem, st>>>(a, p);
 }

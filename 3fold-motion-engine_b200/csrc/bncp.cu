@@ -562,13 +562,10 @@ static int32_t bncp_adjoint(const b2c_bncp *p, int mode, double *dmu, double *db
                             double *gmu, b2c_stream s)
 {
     if (p->n_env == 0) return B2C_OK;
-    static bool attr = false;
     const size_t smem = b2c::bncp::adjoint_smem(p->n_max);
-    if (!attr) {
-        cudaFuncSetAttribute(b2c::bncp::k_adjoint, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)b2c::bncp::adjoint_smem(b2c::bncp::kMaxN));
-        attr = true;
-    }
+    // the opt-in above 48 KB is the device's, so for every launch
+    cudaFuncSetAttribute(b2c::bncp::k_adjoint, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)b2c::bncp::adjoint_smem(b2c::bncp::kMaxN));
     b2c::bncp::k_adjoint<<<p->n_env, 32, smem, b2c::stream_of(s)>>>(p->n_env, p->n_max, p->nc, p->G, p->b, p->mu,
                                                                       p->lam, p->labels, p->status, mode, dmu, db,
                                                                       glam, gb, gmu);

@@ -1089,10 +1089,14 @@ int grid_blocks()
     return n;
 }
 
-// one CTA, a cluster or a cooperative grid of a kernel
+// One CTA, a cluster or a cooperative grid of a kernel.  What a launch opts in to (its shared memory
+// above 48 KB, a cluster above eight CTAs) is the device's, not the process's, so it is set for
+// every launch, and to the kernel's most, so that two threads do not undo each other's.
 int launch_kind(const void *fn, void **args, int kind, int ctas, int threads, size_t smem, const char *what,
                 cudaStream_t s)
 {
+    if (smem > 0) allow_smem(fn, kTableBytes + (kind == kBlock ? kStateBytes : 0));
+    if (kind == kCluster) cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctas);
     cfg.blockDim = dim3(threads);
@@ -1196,9 +1200,8 @@ int sweeps(const b2c_ncp_scene *sc, b2c_ncp_state *st, const b2c_ncp_params *p, 
     if (iters <= 0 || sc->n_c == 0) return B2C_OK;
     SweepArgs<T> a = sweep_args<T>(sc, st, p, iters);
     a.trace = trace;
-    static const bool allowed = allow_smem((const void *)k_sweeps<T, kBlock>, kTableBytes + kStateBytes);
     const size_t state = 6 * (sizeof(T) + 8) * (size_t)sc->n_b;
-    a.smem_bodies = allowed && state <= kStateBytes ? sc->n_b : 0;
+    a.smem_bodies = state <= kStateBytes ? sc->n_b : 0;
     static const PhaseKernel k = {
         {(const void *)k_sweeps<T, kBlock>, (const void *)k_sweeps<T, kCluster>, (const void *)k_sweeps<T, kGrid>},
         {sweep_threads<T, kBlock>(), sweep_threads<T, kCluster>(), sweep_threads<T, kGrid>()},
@@ -1847,8 +1850,6 @@ int adjoint_sweeps(const b2c_ncp_scene *sc, b2c_ncp_state *st, const b2c_ncp_par
     a.timeout_ns = p->barrier_timeout_ns > 0 ? p->barrier_timeout_ns : 1000000000LL;
     cudaMemsetAsync(vb, 0, sizeof(double) * 6 * (size_t)sc->n_b, s);
     if (trace) cudaMemsetAsync(st->res, 0, sizeof(double) * (size_t)sc->n_c, s);
-    static const bool allowed = allow_smem((const void *)k_adj_sweeps<kBlock>, kTableBytes);
-    (void)allowed;
     static const PhaseKernel k = {
         {(const void *)k_adj_sweeps<kBlock>, (const void *)k_adj_sweeps<kCluster>, (const void *)k_adj_sweeps<kGrid>},
         {adj_threads<kBlock>(), adj_threads<kCluster>(), adj_threads<kGrid>()},
