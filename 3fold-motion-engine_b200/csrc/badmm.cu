@@ -307,19 +307,22 @@ __device__ __forceinline__ void pcg(Env<C> &E, const double (&g)[3][3 * C], cons
 // therefore runs every pair with p + q = t (mod M) at once, two sweeps overlapping, and M stages
 // do a sweep's work where the pairs one by one are M (M - 1) / 2 steps.  A stage is a rotation
 // per pair (spread over the problem's lanes), then the 2x2 blocks of the pairs' rows and columns,
-// each one lane's.  It ends early when a whole sweep met no off-diagonal entry above 1e-17 of its
-// diagonal's geometric mean: no eigenvalue can move by a rounding any more.
+// each one lane's.  A problem is done when a whole sweep met none of its off-diagonal entries
+// above 1e-17 of its diagonal's geometric mean: its eigenvalues are then known to a rounding.  It
+// takes no rotation from there on, because two nearly equal diagonal entries still turn by a large
+// angle and can move by that rounding, and a problem's result must not depend on how long its
+// neighbours in the warp go on.
 template <int C>
 __device__ void spectrum(Env<C> &E, int sweeps)
 {
     using D = Dim<C>;
     constexpr int M = D::M;
     double *A = E.A, *cs = E.cs;
-    bool big = false;
+    bool big = false, done = false;
     for (int t = 1; t <= sweeps * M + M - 3; ++t) {
         const int r = t % M, s = t / M;
         const int n1 = r / 2 + 1, K = n1 + (r + M) / 2 - r;  // pairs with p + q = r, and with p + q = r + M
-        for (int k = E.c; k < K; k += D::L) {
+        for (int k = E.c; k < K && !done; k += D::L) {
             const int p = k < n1 ? k : r + 1 + (k - n1), q = k < n1 ? r - p : r + M - p;
             const int sw = k < n1 ? s : s - 1;
             double c = 1.0, sn = 0.0;
@@ -338,7 +341,7 @@ __device__ void spectrum(Env<C> &E, int sweeps)
             cs[2 * k + 1] = sn;
         }
         __syncwarp();
-        for (int P = 0; P < K; ++P) {
+        for (int P = 0; P < K && !done; ++P) {
             const int p = P < n1 ? P : r + 1 + (P - n1), q = P < n1 ? r - p : r + M - p;
             const double cp = cs[2 * P], sp = cs[2 * P + 1];
             for (int Q = E.c; Q < K; Q += D::L) {
@@ -357,7 +360,9 @@ __device__ void spectrum(Env<C> &E, int sweeps)
         }
         __syncwarp();
         if (t % M == 0) {  // stages t - M + 1 .. t met every pair once (from the second window on)
-            if (!__any_sync(kAll, big) && t >= 2 * M) break;
+            const unsigned met = __ballot_sync(kAll, big) >> (E.g * D::L) & ((1u << D::L) - 1u);
+            done = done || (met == 0 && t >= 2 * M);
+            if (__all_sync(kAll, done)) break;
             big = false;
         }
     }
