@@ -25,7 +25,8 @@
 //    from unit sigmas, one (I - B) sigma = a elimination and the response at that sigma, each a
 //    CG solve of the fixed-branch system -- for the direction db = dt J M^-1 e_j (and v+'s
 //    response) and for mu at each problem's first slip contact.  B does not depend on the
-//    direction, so both directions share its columns, and the solves run two at a time.
+//    direction where the CG converges, so both directions share its columns (grad_affine()), and
+//    the solves run two at a time.
 //
 // What bounds it: the CG recurrence's dependent chain (exchange, 3 nc-term row sums, two dot
 // products, one division).  The time per CG step hardly depends on how many problems share a
@@ -682,6 +683,20 @@ __device__ inline void eliminate(double *W, int ld, double *r, double *sig, int 
 
 // grad_affine (NB:1172-1186) for N directions (pinh, db): dlam.  n_calls - 2 columns of B at most
 // (the rest are zero, as the reference's loop leaves them).
+//
+// The reference takes a column of B as the slip speeds' rate with a unit sigma less that without.
+// A solved system is linear, so the column is as well the rate for the unit sigma alone, which
+// every direction shares.  A conjugate gradient that has not converged is not linear in its
+// right-hand side (4 steps at 4 contacts: 0.05 of the gradient), so the short
+// cut is taken from twice the system's rows on (own_columns), where the two forms have agreed to
+// rounding since M steps (batches of 1 to 8 contacts, 6 to 32 coordinates, 2e-13 of the gradient);
+// below, each direction has columns of its own, as the reference forms them.
+template <int C>
+__host__ __device__ constexpr bool own_columns(int cg)
+{
+    return cg < 2 * Dim<C>::M;
+}
+
 template <int C, int N>
 __device__ void grad_affine(Env<C> &E, const Branch &b, const double (&S)[3][3 * C], double mu, double eta,
                             const double (&pinh)[N][3], const double (&db)[N][3], int n_calls, int cg,
@@ -705,7 +720,8 @@ __device__ void grad_affine(Env<C> &E, const Branch &b, const double (&S)[3][3 *
     if (b.lab == 2)
 #pragma unroll
         for (int n = 0; n < N; ++n) E.a[n * C + rank] = so[n];
-    // B's columns: the response of the slip speeds to a unit sigma
+    // B's columns: the response of the slip speeds to a unit sigma (one direction: maybe its own)
+    const bool own = N == 1 && own_columns<C>(cg);
     int most = ns;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(kAll, most, o));
@@ -713,19 +729,20 @@ __device__ void grad_affine(Env<C> &E, const Branch &b, const double (&S)[3][3 *
     for (int i = E.c; i < C * C; i += D::L) E.Bm[i] = 0.0;
     __syncwarp();
     for (int j = 0; j < K && j < most; j += D::R) {
-        double ur[D::R][3], zero[D::R][3], ud[D::R][3], us[D::R];
+        double ur[D::R][3], up[D::R][3], ub[D::R][3], ud[D::R][3], us[D::R];
 #pragma unroll
         for (int n = 0; n < D::R; ++n)
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                zero[n][k] = 0.0;
-                ur[n][k] = k == 0 && b.lab == 2 && rank == j + n ? -mu : 0.0;
+                up[n][k] = own ? pinh[0][k] : 0.0;
+                ub[n][k] = own ? db[0][k] : 0.0;
+                ur[n][k] = (own ? base[0][k] : 0.0) - (k == 0 && b.lab == 2 && rank == j + n ? mu : 0.0);
             }
-        branch_solve<C, D::R>(E, b, S, eta, ur, zero, zero, cg, ud, us);
+        branch_solve<C, D::R>(E, b, S, eta, ur, up, ub, cg, ud, us);
         if (b.lab == 2)
 #pragma unroll
             for (int n = 0; n < D::R; ++n)
-                if (j + n < ns && j + n < K) E.Bm[rank * C + j + n] = us[n];
+                if (j + n < ns && j + n < K) E.Bm[rank * C + j + n] = own ? us[n] - so[0] : us[n];
     }
     __syncwarp();
     if (E.c == 0) {
@@ -900,7 +917,7 @@ __global__ void __launch_bounds__(32, C <= 5 ? 8 : 4) k_admm(b2c_admm P, b2c_adm
     const int dirs = !given && prm.do_mu ? 2 : 1;
     int done = 0;
     if constexpr (D::R == 2) {
-        if (dirs == 2) {
+        if (dirs == 2 && !own_columns<C>(prm.grad_cg)) {
             double pin[2][3], db[2][3], dl[2][3];
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
