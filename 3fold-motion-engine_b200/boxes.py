@@ -258,7 +258,8 @@ class BoxContactEngine(_BeadEngineBase):
     def color_cache_misses(self):
         return int(self.p_bufs["cache_state"][4].item()) if self._built else 0
 
-    # staged substep with CUDA events (profiling); same launches as b2c_box_substep
+    # staged substep with CUDA events (profiling); same launches as b2c_box_substep, but the
+    # candidates' emission searches again (there the contact slots keep the partners for it)
     STAGES = ("predict", "candidates", "narrowphase", "colour", "solve", "warm_store", "integrate")
 
     def profile_substep(self, dt):

@@ -199,9 +199,9 @@ __device__ __forceinline__ int group_collect(bool on, int i, const float *__rest
 
 // The search is the broadphase's cost, so it runs once where the partners can be kept until the
 // emission: `list`, kMaxBoxCandidates words a body, in the contact slots that the narrowphase
-// overwrites later (NULL: count only, and the emission searches again).  Measured on a
-// B200, count + emission in us, a warp a body with remainders for the wraps and two searches
-// before: 100 000 cubes 72 + 82 -> 57 + 16, a pile of 10 000 boxes 20 + 21 -> 17 + 3.5.
+// overwrites later (NULL: count only, and the emission searches again; box_candidates()).
+// Measured on a B200, count + emission in us, a warp a body with remainders for the wraps and two
+// searches before: 100 000 cubes 72 + 82 -> 57 + 16, a pile of 10 000 boxes 20 + 21 -> 17 + 3.5.
 __global__ void __launch_bounds__(kBroadLanes * kBroadBodies)
     k_box_cand_count(int n, const float *__restrict__ xc, const float *__restrict__ half,
                      const int *__restrict__ start, const int *__restrict__ sorted, BoxGrid g, float margin,
@@ -386,7 +386,9 @@ static BoxGrid box_grid_of(const b2c_boxes *bx)
                    1.0f / bx->cell, bx->scene};
 }
 
-int box_candidates(const b2c_bodies *b, b2c_boxes *bx, b2c_header *hdr, cudaStream_t s)
+// slots_free: the narrowphase follows and overwrites the contact slots, so they can keep the partners
+// meanwhile.  A caller of the candidates alone may still read the last narrowphase's slots.
+int box_candidates(const b2c_bodies *b, b2c_boxes *bx, b2c_header *hdr, bool slots_free, cudaStream_t s)
 {
     const int n = b->n;
     const int nbk = bx->dim_x * bx->dim_y * bx->dim_z;
@@ -400,7 +402,7 @@ int box_candidates(const b2c_bodies *b, b2c_boxes *bx, b2c_header *hdr, cudaStre
     if (n > 0) k_box_scatter<<<blocks_for(n), kThreads, 0, s>>>(n, bx->bucket, bx->start, bx->cursor, bx->sorted);
     const int bgrid = std::max(1, (n + kBroadBodies - 1) / kBroadBodies), bt = kBroadLanes * kBroadBodies;
     // a candidate's eight contact slots are 32 words: room for kMaxBoxCandidates words a body
-    int *list = bx->slot_p && (long long)bx->cand_capacity * kSlots * 4 >= (long long)n * kMaxBoxCandidates
+    int *list = slots_free && (long long)bx->cand_capacity * kSlots * 4 >= (long long)n * kMaxBoxCandidates
                     ? reinterpret_cast<int *>(bx->slot_p) : nullptr;
     k_box_cand_count<<<bgrid, bt, 0, s>>>(n, b->xc, bx->half, bx->start, bx->sorted, g, bx->margin, bx->cand_count, list,
                                           hdr);
@@ -478,7 +480,7 @@ extern "C" int32_t b2c_box_candidates(const b2c_bodies *b, b2c_boxes *bx, b2c_he
         b2c::set_error("b2c_box_candidates: bad argument");
         return B2C_EARG;
     }
-    return b2c::box_candidates(b, bx, hdr, b2c::stream_of(s));
+    return b2c::box_candidates(b, bx, hdr, false, b2c::stream_of(s));
 }
 
 extern "C" int32_t b2c_box_contacts(const b2c_bodies *b, b2c_boxes *bx, b2c_contacts *kept, int64_t *kept_keys,
@@ -504,7 +506,7 @@ extern "C" int32_t b2c_box_substep(const b2c_bodies *b, b2c_boxes *bx, b2c_conta
     cudaStream_t st = b2c::stream_of(s);
     int rc;
     if ((rc = b2c::body_predict_substep(b, dt, vgrav, true, st))) return rc;
-    if ((rc = b2c::box_candidates(b, bx, hdr, st))) return rc;
+    if ((rc = b2c::box_candidates(b, bx, hdr, true, st))) return rc;
     if ((rc = b2c::box_contacts(b, bx, kept, kept_keys, pr, warm, hdr, p, st))) return rc;
     if ((rc = b2c::color_pairs(b, pr, hdr, p, st))) return rc;
     if ((rc = b2c::color_solve(b, kept, pr, hdr, p, dt, st))) return rc;

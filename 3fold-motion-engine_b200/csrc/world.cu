@@ -25,7 +25,7 @@
 namespace b2c {
 
 int exclusive_scan(const int *in, int *out, int n, const int *dn, int *scratch, cudaStream_t s);
-int box_candidates(const b2c_bodies *b, b2c_boxes *bx, b2c_header *hdr, cudaStream_t s);
+int box_candidates(const b2c_bodies *b, b2c_boxes *bx, b2c_header *hdr, bool slots_free, cudaStream_t s);
 
 namespace world {
 
@@ -680,7 +680,7 @@ extern "C" int32_t b2c_world_contacts(b2c_world *wd, b2c_boxes *bx, b2c_header *
     b2c_bodies mirror{};
     mirror.n = n;
     mirror.xc = wd->xc32;
-    int rc = box_candidates(&mirror, bx, hdr, s);
+    int rc = box_candidates(&mirror, bx, hdr, false, s);
     if (rc) return rc;
     const int cgrid = std::min(blocks_for(cap, 128), kSMs * 16);
     k_narrow<<<cgrid, 128, 0, s>>>(bx->cand_offset, n, cap, bx->cand_a, bx->cand_b, wd->x4, wd->q, wd->half4,

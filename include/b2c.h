@@ -238,7 +238,8 @@ typedef struct b2c_boxes {
     int32_t *cont_offset;     /* (cand cap+1) */
     int32_t *pair_flag;       /* (cand cap+1) 1 when the candidate has contacts */
     int32_t *pair_offset;     /* (cand cap+1) */
-    float *slot_p;            /* (cand cap x 8, 4) contact point | gap */
+    float *slot_p;            /* (cand cap x 8, 4) contact point | gap (within b2c_box_substep also
+                                 the broadphase's scratch) */
     float *slot_n;            /* (cand cap, 4) normal from b to a */
     int32_t *slot_f;          /* (cand cap x 8) feature id */
     int32_t *scan_tmp;        /* b2c_scan_scratch_ints(max(dims, n, cand cap) + 1) */
