@@ -827,13 +827,20 @@ __global__ void __launch_bounds__(kColorThreads) k_color_pairs(b2c_header *hdr, 
     cluster.sync();  // every CTA's counts stay alive until the others are done reading them
 }
 
+// What a colouring launch opts in to, a cluster above eight CTAs and shared memory above 48 KB, is the
+// device's and not the process's, so it is set for every launch.
+static void allow_color_launch()
+{
+    cudaFuncSetAttribute(k_color_pairs, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaFuncSetAttribute(k_color_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, kColorDynSmem);
+}
+
 // largest power-of-two cluster (<= 16) of colouring CTAs the device co-schedules; cached
 static int color_cluster_size()
 {
     static int cached = -1;
     if (cached < 0) {
-        cudaFuncSetAttribute(k_color_pairs, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        cudaFuncSetAttribute(k_color_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, kColorDynSmem);
+        allow_color_launch();
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(kColorClusterMax);
         cfg.blockDim = dim3(kColorThreads);
@@ -966,6 +973,7 @@ int color_pairs(const b2c_bodies *b, b2c_pairs *pr, b2c_header *hdr, const b2c_c
         return B2C_EARG;
     }
     const int cs = color_cluster_size();
+    allow_color_launch();
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(cs);
     cfg.blockDim = dim3(kColorThreads);

@@ -1267,22 +1267,12 @@ int island_partition_engine(const b2c_bodies *b, b2c_pairs *pr, b2c_header *hdr,
 // dynamic shared memory of a solve launch: the contact staging of its threads
 static size_t stage_bytes(int threads) { return (size_t)kStageBytesPerThread * threads; }
 
-// the solve kernels' dynamic shared memory exceeds the 48 KB default: opt in once
-static void allow_stage_smem()
+// What a solve launch opts in to, shared memory above 48 KB and clusters above eight CTAs, is the
+// device's and not the process's, so it is set for every launch.
+static void allow(const void *fn, int threads, bool cluster = false)
 {
-    static bool done = false;
-    if (done) return;
-    cudaFuncSetAttribute(k_color_solve_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage_bytes(256));
-    cudaFuncSetAttribute(k_color_solve_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage_bytes(256));
-    cudaFuncSetAttribute(k_color_solve_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)stage_bytes(kClusterThreads));
-    cudaFuncSetAttribute(k_color_solve_cluster_row, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)stage_bytes(kClusterThreadsRow));
-    cudaFuncSetAttribute(k_color_solve_scenes, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)stage_bytes(kSceneThreads));
-    cudaFuncSetAttribute(k_island_solve, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)stage_bytes(kIslandThreads));
-    done = true;
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage_bytes(threads));
+    if (cluster) cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
 }
 
 static int max_coresident_grid_blocks()
@@ -1292,7 +1282,7 @@ static int max_coresident_grid_blocks()
         int dev = 0, sms = 0, per = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        allow_stage_smem();
+        allow((const void *)k_color_solve_grid, 256);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_color_solve_grid, 256, stage_bytes(256));
         cached = std::min(kBarrierMaxCTAs, std::max(1, sms * std::max(per, 1)));
     }
@@ -1307,8 +1297,7 @@ static int max_cluster_size(int row)
     static int cached[2] = {-1, -1};
     if (cached[row] < 0) {
         const void *fn = row ? (const void *)k_color_solve_cluster_row : (const void *)k_color_solve_cluster;
-        cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        allow_stage_smem();
+        allow(fn, row ? kClusterThreadsRow : kClusterThreads, true);
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(kClusterMax);
         cfg.blockDim = dim3(row ? kClusterThreadsRow : kClusterThreads);
@@ -1390,14 +1379,14 @@ int color_solve(const b2c_bodies *b, b2c_contacts *kept, b2c_pairs *pr, b2c_head
     if (islands) {
         const int *isl_slots = nullptr, *isl_at = nullptr;
         if ((rc = island_partition_engine(b, pr, hdr, &a.island_info, &isl_slots, &isl_at, s))) return rc;
-        allow_stage_smem();
+        allow((const void *)k_island_solve, kIslandThreads);
         k_island_solve<<<std::min(blocks_for(2LL * pr->capacity + 32, kIslandThreads), kSMs * 4), kIslandThreads,
                          stage_bytes(kIslandThreads), s>>>(a, isl_slots, isl_at);
         if ((rc = check_launch("island_solve"))) return rc;
     }
     int mode = p->solve_blocks;
     if (scenes) {
-        allow_stage_smem();
+        allow((const void *)k_color_solve_scenes, kSceneThreads);
         const SceneSched sc{pr->pbi, pr->col, pr->scene_body_start, pr->scene_order, pr->pair_slot,
                             pr->scene_slots};
         k_color_solve_scenes<<<pr->n_scenes, kSceneThreads, stage_bytes(kSceneThreads), s>>>(a, sc);
@@ -1424,6 +1413,8 @@ int color_solve(const b2c_bodies *b, b2c_contacts *kept, b2c_pairs *pr, b2c_head
             attr[0].val.clusterDim.z = 1;
             cfg.attrs = attr;
             cfg.numAttrs = 1;
+            allow(a.row ? (const void *)k_color_solve_cluster_row : (const void *)k_color_solve_cluster,
+                  a.row ? kClusterThreadsRow : kClusterThreads, true);
             cudaError_t e = a.row ? cudaLaunchKernelEx(&cfg, k_color_solve_cluster_row, a)
                                   : cudaLaunchKernelEx(&cfg, k_color_solve_cluster, a);
             if (e != cudaSuccess) {
@@ -1437,9 +1428,9 @@ int color_solve(const b2c_bodies *b, b2c_contacts *kept, b2c_pairs *pr, b2c_head
         }
     }
     if (mode > 0) {
-        allow_stage_smem();
         const int nblocks = std::max(1, std::min(mode, max_coresident_grid_blocks()));
         if (nblocks == 1) {
+            allow((const void *)k_color_solve_block, 256);
             k_color_solve_block<<<1, 256, stage_bytes(256), s>>>(a);
             if ((rc = check_launch("color_solve_block"))) return rc;
         } else {
@@ -1454,6 +1445,7 @@ int color_solve(const b2c_bodies *b, b2c_contacts *kept, b2c_pairs *pr, b2c_head
             attr[0].val.cooperative = 1;
             cfg.attrs = attr;
             cfg.numAttrs = 1;
+            allow((const void *)k_color_solve_grid, 256);
             cudaError_t e = cudaLaunchKernelEx(&cfg, k_color_solve_grid, a);
             if (e != cudaSuccess) {
                 set_error("color_solve: cooperative launch of %d blocks: %s", nblocks, cudaGetErrorString(e));
