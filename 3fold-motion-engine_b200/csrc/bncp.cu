@@ -22,6 +22,8 @@
 //
 // Sums run in a fixed order that padding with empty contacts does not change, so results are
 // bit-identical run to run and whatever a batch is padded to.
+#include <type_traits>
+
 #include "b2c_common.cuh"
 
 namespace b2c {
@@ -123,6 +125,12 @@ struct Lanes {
 // (the slowest problem's 940 sweeps); at B = 4096, 1 contact 107 -> 28 us, 8 contacts 20.0 ->
 // 4.9 ms.  Error of lambda against 80-bit arithmetic, same sweeps: 1 contact 1.2e-16 -> 1.1e-16 of
 // its norm, 4 contacts 2.5e-16 -> 2.2e-16.
+//
+// Above 8 contacts the rows come from shared memory, whose bandwidth bounds a full SM, so a
+// problem's rows have its batch's length, only the lane whose turn it is reads its own, and a warp
+// stops at its own problems' contacts.  100 sweeps of 4 096 problems, us, a warp a problem before:
+// 9 contacts 1 502 -> 1 006, 12 3 346 -> 1 990, 16 6 136 -> 4 515, 1 to 16 at random 3 990 -> 4 150;
+// padded, 1 contact each in a batch of 8: 192 -> 125.
 template <int C>
 __global__ void __launch_bounds__(32) k_solve(int n_env, int n_max, const int *__restrict__ ncs,
                                               const double *__restrict__ G, const double *__restrict__ b,
@@ -135,10 +143,14 @@ __global__ void __launch_bounds__(32) k_solve(int n_env, int n_max, const int *_
     extern __shared__ double sm[];
     const int lane = (int)(threadIdx.x & 31), pg = lane / D::L, me = lane % D::L;
     const int e = (int)blockIdx.x * D::PW + pg, ec = e < n_env ? e : n_env - 1;
-    const int nc = ncs[ec], ncm = n_max / 3;
+    const int ncm = n_max / 3, nc = min(ncs[ec], ncm);
     const bool own = me < nc;
     const double *Ge = G + (size_t)ec * n_max * n_max;
     double *Gs = sm + (size_t)pg * (M * D::S + M), *xs = Gs + M * D::S;  // kRegs: not used
+    // the most contacts of a problem of the warp: above 8 its turns and rows end there; up to 8, where
+    // it is a third of C or less (a batch of padded problems), there are only so many turns.  A
+    // reduction, not shuffles: the branches on it are then known to be the same for the whole warp.
+    const int cm = __reduce_max_sync(0xffffffffu, nc);
     double g[3][R], x[R], bb[3] = {0.0, 0.0, 0.0}, rho = 0.0, m = 0.0;
     if (D::kRegs) {
 #pragma unroll
@@ -181,12 +193,30 @@ __global__ void __launch_bounds__(32) k_solve(int n_env, int n_max, const int *_
             }
         } else {
             const double *r0 = Gs + 3 * (me < C ? me : 0) * D::S;
-            for (int q = 0; q < C; ++q) {
-                const int c = first + q < C ? first + q : first + q - C, j = 3 * c;
-                for (int k = 0; k < 3; ++k) {
-                    const double *r = r0 + k * D::S;
-                    u[k] = fma(r[j + 2], xs[j + 2], fma(r[j + 1], xs[j + 1], fma(r[j], xs[j], u[k])));
+            auto part = [&](int from, int to) {
+#pragma unroll 4
+                for (int c = from; c < to; ++c) {
+                    const int j = 3 * c;
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) {
+                        const double *r = r0 + k * D::S;
+                        u[k] = fma(r[j + 2], xs[j + 2], fma(r[j + 1], xs[j + 1], fma(r[j], xs[j], u[k])));
+                    }
                 }
+            };
+            if (cm == C) {  // the bound known when compiled: 1.3 times as fast at 16 contacts
+#pragma unroll
+                for (int q = 0; q < C; ++q) {
+                    const int c = first + q < C ? first + q : first + q - C, j = 3 * c;
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) {
+                        const double *r = r0 + k * D::S;
+                        u[k] = fma(r[j + 2], xs[j + 2], fma(r[j + 1], xs[j + 1], fma(r[j], xs[j], u[k])));
+                    }
+                }
+            } else {
+                part(first, cm);
+                part(0, first);
             }
         }
     };
@@ -213,36 +243,44 @@ __global__ void __launch_bounds__(32) k_solve(int n_env, int n_max, const int *_
     bool run = e < n_env;
     double res = 0.0;
     int iters = max_iters;
-    for (int it = 0; it < max_iters; ++it) {
-        if (check > 0 && it % check == 0) {
-            const double r = residual();
-            if (run) {
-                res = r;
-                if (r < tol) {
-                    run = false;
-                    iters = it;
+    // the sweeps, over T turns (in shared memory cm)
+    auto sweeps = [&](auto turns) {
+        constexpr int T = decltype(turns)::value;
+        for (int it = 0; it < max_iters; ++it) {
+            if (check > 0 && it % check == 0) {
+                const double r = residual();
+                if (run) {
+                    res = r;
+                    if (r < tol) {
+                        run = false;
+                        iters = it;
+                    }
                 }
+                if (!__any_sync(0xffffffffu, run)) break;
             }
-            if (!__any_sync(0xffffffffu, run)) break;
-        }
 #pragma unroll U
-        for (int c = 0; c < C; ++c) {
-            double u[3], out[3], lo[3];
-            rows(c, u);
+            for (int c = 0; c < (D::kRegs ? T : cm); ++c) {
+                double u[3], out[3], lo[3];
+                if (D::kRegs || me == c) {  // in shared memory the other lanes' rows would only cost its bandwidth
+                    rows(c, u);
 #pragma unroll
-            for (int k = 0; k < 3; ++k) lo[k] = D::kRegs ? x[(3 * c + k) % R] : xs[3 * c + k];
-            update(u, lo, m, rho, den, iden, out);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const double v = __shfl_sync(0xffffffffu, out[k], c, D::L);
-                if (run && c < nc) {
-                    if (D::kRegs) x[(3 * c + k) % R] = v;
-                    else if (me == 0) xs[3 * c + k] = v;
+                    for (int k = 0; k < 3; ++k) lo[k] = D::kRegs ? x[(3 * c + k) % R] : xs[3 * c + k];
+                    update(u, lo, m, rho, den, iden, out);
                 }
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const double v = __shfl_sync(0xffffffffu, out[k], c, D::L);
+                    if (run && c < nc) {
+                        if (D::kRegs) x[(3 * c + k) % R] = v;
+                        else if (me == 0) xs[3 * c + k] = v;
+                    }
+                }
+                if (!D::kRegs) __syncwarp();
             }
-            if (!D::kRegs) __syncwarp();
         }
-    }
+    };
+    if (D::kRegs && 3 * cm <= C) sweeps(std::integral_constant<int, C / 3>{});
+    else sweeps(std::integral_constant<int, C>{});
     if (__any_sync(0xffffffffu, run)) {  // the residual of the final iterate
         const double r = residual();
         if (run) res = r;
@@ -554,6 +592,13 @@ extern "C" int32_t b2c_bncp_solve(const b2c_bncp *p, int32_t max_iters, double t
         case 6: return b2c::bncp::solve<6>(p, max_iters, tol, check, st);
         case 7: return b2c::bncp::solve<7>(p, max_iters, tol, check, st);
         case 8: return b2c::bncp::solve<8>(p, max_iters, tol, check, st);
+        case 9: return b2c::bncp::solve<9>(p, max_iters, tol, check, st);
+        case 10: return b2c::bncp::solve<10>(p, max_iters, tol, check, st);
+        case 11: return b2c::bncp::solve<11>(p, max_iters, tol, check, st);
+        case 12: return b2c::bncp::solve<12>(p, max_iters, tol, check, st);
+        case 13: return b2c::bncp::solve<13>(p, max_iters, tol, check, st);
+        case 14: return b2c::bncp::solve<14>(p, max_iters, tol, check, st);
+        case 15: return b2c::bncp::solve<15>(p, max_iters, tol, check, st);
         default: return b2c::bncp::solve<16>(p, max_iters, tol, check, st);
     }
 }
