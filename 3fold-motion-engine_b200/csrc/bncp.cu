@@ -471,7 +471,19 @@ __device__ void lu_solve_t(const double *A, const int *piv, int n, double *y, in
     __syncwarp();
 }
 
+// A warp's matrices are sized by the batch's largest problem, C contacts: at 4 contacts 4.2 KB, so 32
+// warps fit an SM where the 64 KB of a 16-contact problem let three (4096 problems: 285 -> 56 us).
+// C is a template parameter because the matrices' places are then known when the kernel is
+// compiled (a place worked out from n_max cost a batch of 16 problems 3 to 4 %, 8 contacts
+// 71.8 -> 74.9 us).
+template <int C>
+constexpr size_t adjoint_smem()
+{
+    return sizeof(double) * (27 * C * C + 3 * C * C + 9 * C + C);
+}
+
 // mode 0: full responses dlam/dmu (n x nc) and dlam/db (n x n); mode 1: vector-Jacobian product
+template <int C>
 __global__ void __launch_bounds__(32) k_adjoint(int n_env, int n_max, const int *__restrict__ ncs,
                                                 const double *__restrict__ G, const double *__restrict__ b,
                                                 const double *__restrict__ mu, const double *__restrict__ lam_in,
@@ -484,8 +496,9 @@ __global__ void __launch_bounds__(32) k_adjoint(int n_env, int n_max, const int 
     const int e = blockIdx.x, lane = threadIdx.x;
     if (e >= n_env) return;
     const int nc = ncs[e], n = 3 * nc, ncm = n_max / 3;
-    double *Gs = sm, *A = Gs + n_max * n_max, *Bb = A + n_max * n_max, *Bmu = Bb + n_max * n_max;
-    double *bs = Bmu + n_max * ncm, *lam = bs + n_max, *mus = lam + n_max, *y = mus + ncm;
+    constexpr int N = 3 * C;
+    double *Gs = sm, *A = Gs + N * N, *Bb = A + N * N, *Bmu = Bb + N * N;
+    double *bs = Bmu + N * C, *lam = bs + N, *mus = lam + N, *y = mus + C;
     __shared__ int piv[kMaxN];
     __shared__ int labels[kMaxN / 3];
     const double *Ge = G + (size_t)e * n_max * n_max;
@@ -546,14 +559,6 @@ __global__ void __launch_bounds__(32) k_adjoint(int n_env, int n_max, const int 
     }
 }
 
-// A warp's matrices, sized by the batch's largest problem: at 4 contacts 4.2 KB, so 32 warps
-// fit an SM where the 64 KB of a 16-contact problem let three (4096 problems: 285 -> 56 us).
-size_t adjoint_smem(int n_max)
-{
-    const size_t n = n_max, c = n_max / 3;
-    return sizeof(double) * (3 * n * n + n * c + 3 * n + c);
-}
-
 template <int C>
 int32_t solve(const b2c_bncp *p, int max_iters, double tol, int check, cudaStream_t st)
 {
@@ -562,6 +567,17 @@ int32_t solve(const b2c_bncp *p, int max_iters, double tol, int check, cudaStrea
     k_solve<C><<<(p->n_env + D::PW - 1) / D::PW, 32, smem, st>>>(p->n_env, p->n_max, p->nc, p->G, p->b, p->mu, p->lam,
                                                                   p->res, p->iters, max_iters, tol, check);
     return check_launch("bncp_solve");
+}
+
+template <int C>
+int32_t adjoint(const b2c_bncp *p, int mode, double *dmu, double *db, const double *glam, double *gb, double *gmu,
+                cudaStream_t st)
+{
+    // the opt-in above 48 KB is the device's, so for every launch
+    cudaFuncSetAttribute(k_adjoint<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)adjoint_smem<C>());
+    k_adjoint<C><<<p->n_env, 32, adjoint_smem<C>(), st>>>(p->n_env, p->n_max, p->nc, p->G, p->b, p->mu, p->lam,
+                                                          p->labels, p->status, mode, dmu, db, glam, gb, gmu);
+    return check_launch("bncp_adjoint");
 }
 
 }  // namespace bncp
@@ -607,14 +623,28 @@ static int32_t bncp_adjoint(const b2c_bncp *p, int mode, double *dmu, double *db
                             double *gmu, b2c_stream s)
 {
     if (p->n_env == 0) return B2C_OK;
-    const size_t smem = b2c::bncp::adjoint_smem(p->n_max);
-    // the opt-in above 48 KB is the device's, so for every launch
-    cudaFuncSetAttribute(b2c::bncp::k_adjoint, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)b2c::bncp::adjoint_smem(b2c::bncp::kMaxN));
-    b2c::bncp::k_adjoint<<<p->n_env, 32, smem, b2c::stream_of(s)>>>(p->n_env, p->n_max, p->nc, p->G, p->b, p->mu,
-                                                                      p->lam, p->labels, p->status, mode, dmu, db,
-                                                                      glam, gb, gmu);
-    return b2c::check_launch("bncp_adjoint");
+    const cudaStream_t st = b2c::stream_of(s);
+    switch (p->n_max / 3) {
+#define B2C_BNCP_CASE(c) \
+    case c: return b2c::bncp::adjoint<c>(p, mode, dmu, db, glam, gb, gmu, st);
+        B2C_BNCP_CASE(1)
+        B2C_BNCP_CASE(2)
+        B2C_BNCP_CASE(3)
+        B2C_BNCP_CASE(4)
+        B2C_BNCP_CASE(5)
+        B2C_BNCP_CASE(6)
+        B2C_BNCP_CASE(7)
+        B2C_BNCP_CASE(8)
+        B2C_BNCP_CASE(9)
+        B2C_BNCP_CASE(10)
+        B2C_BNCP_CASE(11)
+        B2C_BNCP_CASE(12)
+        B2C_BNCP_CASE(13)
+        B2C_BNCP_CASE(14)
+        B2C_BNCP_CASE(15)
+#undef B2C_BNCP_CASE
+        default: return b2c::bncp::adjoint<16>(p, mode, dmu, db, glam, gb, gmu, st);
+    }
 }
 
 extern "C" int32_t b2c_bncp_sensitivity(const b2c_bncp *p, double *dlam_dmu, double *dlam_db, b2c_stream s)
