@@ -84,7 +84,7 @@ struct SolveArgs {
     unsigned int *bar_count;  // the grid barrier's arrival counter
     long long timeout_ns;
     const int *island_info;   // the island partition's statistics (B2C_COLOR_ISLANDS) or NULL
-    int choose;               // the cluster and the grid are both launched: the colouring decides
+    int choose;               // > 0: cluster and grid are both launched, the grid runs from so many pairs a colour
 };
 
 // The island solve ran this substep (its partition has no island above B2C_ISLAND_MAX_PAIRS
@@ -103,8 +103,9 @@ __global__ void k_pair_gather(const b2c_header *__restrict__ hdr, const int *__r
                               const int *__restrict__ pidx, const int *__restrict__ pbi, const int *__restrict__ pbj,
                               b2c_contacts kept, const float *__restrict__ xc, const float *__restrict__ invIw,
                               const float *__restrict__ invM, const float *__restrict__ body_mu, float mu, Records R,
-                              b2c_header *hdr_w)
+                              b2c_header *hdr_w, unsigned int *arrivals)
 {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *arrivals = 0;  // the grid solve's barrier starts from zero
     const int P = (hdr->n_pairs > 0 && hdr->n_colors > 0) ? hdr->n_pairs : 0;
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < P; s += gridDim.x * blockDim.x) {
         const int p = porder[s];
@@ -182,8 +183,9 @@ __global__ void k_pair_gather_row(const b2c_header *__restrict__ hdr, const int 
                                   const float *__restrict__ invIw, const float *__restrict__ invM,
                                   const float *__restrict__ body_mu, float mu, float dt, Records R, b2c_header *hdr_w,
                                   const int *__restrict__ col, int *__restrict__ body_slots,
-                                  int *__restrict__ pair_slot)
+                                  int *__restrict__ pair_slot, unsigned int *arrivals)
 {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *arrivals = 0;  // the grid solve's barrier starts from zero
     const int P = (hdr->n_pairs > 0 && hdr->n_colors > 0) ? hdr->n_pairs : 0;
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < P; s += gridDim.x * blockDim.x) {
         const int p = porder[s];
@@ -947,16 +949,18 @@ __device__ void pair_position_row(const SolveArgs &a, int s, const BA &B, const 
 // ---------------------------------------------------------------------------------------------
 constexpr int kMaxSolveColors = 512;  // the colouring's cap (kMaxColorsCap)
 
-// The automatic form of a scene of kWidePairs bodies or more is decided on the device, by the
-// pairs of a colour: both the 16-CTA cluster and the grid of every SM are launched (the one that
-// is not wanted returns at once, ~2 us), because the colouring is not known when a captured step
-// is launched.  Narrow colours are latency, and the cluster's barrier is the cheaper one (0.25
-// against 1.3 us); a colour that fills the cluster's warps loops on its 16 SMs.  Measured on a
-// B200, cluster / grid in us per step of two substeps (bead lattice: one): 516 pairs a colour (pile
-// of 3 000 boxes) 1 915 / 2 149; 1 500 (bead lattice of 3 000) 540 / 573; 1 767 (20 000 cubes)
-// 1 277 / 1 171; 1 860 (pile of 10 000) 2 470 / 2 413; 2 390 (160 piles, 67 000 boxes) 2 373 /
-// 2 057; 5 000 (bead lattice of 10 000) 739 / 600; 8 680 (100 000 cubes) 3 275 / 1 813.
-constexpr int kWidePairs = 1700;
+// The automatic form of a scene of twice that many bodies is decided on the device, by the pairs of a
+// colour: both the 16-CTA cluster and the grid of every SM are launched (the one that is not
+// wanted returns at once, ~5 us), because the colouring is not known when a captured step is
+// launched; a smaller scene has such colours only where there are one or two of them.  Narrow
+// colours are latency, and the cluster's barrier is the cheaper one (0.25 against 1.3 us); a colour
+// that fills the cluster's warps loops on its 16 SMs, in the row form from fewer pairs on.  Measured
+// on a B200, cluster / grid in us per step.  Row form, two substeps: 1 058 pairs a colour (12 000
+// cubes) 1 032 / 1 095; 1 270 (pile of 8 000 boxes) 2 421 / 2 488; 1 701 (pile of 10 000) 2 475 /
+// 2 427; 1 772 (20 000 cubes) 1 204 / 1 110; 2 390 (160 piles, 67 000 boxes) 2 373 / 2 057; 8 680
+// (100 000 cubes) 3 275 / 1 813.  Reference form, bead lattices of two colours, one substep: 1 700
+// 534 / 564; 2 300 542 / 552; 2 600 560 / 566; 3 000 587 / 594; 3 500 669 / 578; 5 000 739 / 600.
+constexpr int kWidePairsRow = 1700, kWidePairs = 3100;
 
 // The phases of the persistent solve (both forms).  Task layout of a colour of cnt pairs: velocity (or warm) tasks
 // [0, cnt) and position tasks [P0, P0 + cnt) with P0 = cnt rounded up to a warp, in every pass
@@ -972,7 +976,7 @@ __device__ __forceinline__ void solve_phases(const SolveArgs &a, const BA &B)
 {
     const int nc = a.hdr->n_colors;
     if (a.hdr->n_pairs == 0 || nc == 0 || islands_took_solve(a)) return;  // uniform over all CTAs
-    if (a.choose && (kKind == kGrid) != (a.hdr->n_pairs >= (long long)kWidePairs * nc)) return;
+    if (a.choose && (kKind == kGrid) != (a.hdr->n_pairs >= (long long)a.choose * nc)) return;
     __shared__ int s_cstart[kMaxSolveColors], s_ccount[kMaxSolveColors];
     for (int c = threadIdx.x; c < nc && c < kMaxSolveColors; c += blockDim.x) {
         s_cstart[c] = a.cstart[c];
@@ -1362,10 +1366,11 @@ int color_solve(const b2c_bodies *b, b2c_contacts *kept, b2c_pairs *pr, b2c_head
         k_pair_gather_row<<<pgrid, kThreads, 0, s>>>(hdr, pr->porder, pr->pstart, pr->kcount, pr->pidx, pr->pbi,
                                                      pr->pbj, *kept, b->xc, b->invIw, b->invM, p->body_mu, p->mu, dt,
                                                      a.rec, hdr, pr->col, warm_bodies ? pr->body_slots : nullptr,
-                                                     scenes ? pr->pair_slot : nullptr);
+                                                     scenes ? pr->pair_slot : nullptr, a.bar_count);
     else
         k_pair_gather<<<pgrid, kThreads, 0, s>>>(hdr, pr->porder, pr->pstart, pr->kcount, pr->pidx, pr->pbi, pr->pbj,
-                                                 *kept, b->xc, b->invIw, b->invM, p->body_mu, p->mu, a.rec, hdr);
+                                                 *kept, b->xc, b->invIw, b->invM, p->body_mu, p->mu, a.rec, hdr,
+                                                 a.bar_count);
     int rc = check_launch("pair_gather");
     if (rc) return rc;
     if (warm_bodies) {
@@ -1399,8 +1404,8 @@ int color_solve(const b2c_bodies *b, b2c_contacts *kept, b2c_pairs *pr, b2c_head
     if (mode < 0) {
         const int cs = std::min(-mode, max_cluster_size(a.row));
         if (cs >= 2) {
-            // a colour has at most n pairs, so below kWidePairs bodies the cluster always runs
-            a.choose = p->solve_blocks == 0 && !scenes && b->n >= kWidePairs && max_coresident_grid_blocks() > cs;
+            const int wide = a.row ? kWidePairsRow : kWidePairs;
+            if (p->solve_blocks == 0 && !scenes && b->n >= 2 * wide && max_coresident_grid_blocks() > cs) a.choose = wide;
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(cs);
             cfg.blockDim = dim3(a.row ? kClusterThreadsRow : kClusterThreads);
@@ -1434,7 +1439,6 @@ int color_solve(const b2c_bodies *b, b2c_contacts *kept, b2c_pairs *pr, b2c_head
             k_color_solve_block<<<1, 256, stage_bytes(256), s>>>(a);
             if ((rc = check_launch("color_solve_block"))) return rc;
         } else {
-            cudaMemsetAsync(a.bar_count, 0, sizeof(uint32_t), s);  // the arrival count restarts every launch
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(nblocks);
             cfg.blockDim = dim3(256);
