@@ -36,8 +36,6 @@ constexpr double kScale = 1.0e10;
 constexpr int kColorThreads = 1024;
 constexpr int kClusterMax = 16;
 constexpr int kMaxColors = 1024;  // the reference's _NCOLMAX
-constexpr int kNarrow = 16;           // contacts a colour, on average, below which one CTA runs the sweeps,
-constexpr int kNarrowContacts = 2048; // of at most this many contacts
 
 enum Stat { kNColors = 0, kCacheValid = 1, kCachedC = 2, kCacheHit = 3, kHits = 4, kMisses = 5, kRounds = 6,
             kError = 7 };
@@ -272,14 +270,19 @@ enum Kind { kBlock = 0, kCluster = 1, kGrid = 2 };
 // colour 1.5 / 2.0 / 3.2, 22 2.4 / 2.0 / 3.2, 85 7.3 / 2.1 / 3.2, 300 24 / 2.3 / 3.3, 400 - / 4.3 / 3.4,
 // 5 000 - / 31 / 4.4.  In float32 the cluster has 640 groups and crosses at 500 to 600.
 struct Form {
-    int asked;  // 0 auto: the launched kernels choose by the colouring; else every launch runs
-    int wide;   // contacts a colour, on average, from which the grid runs
-    __device__ __forceinline__ bool here(int kind, int nc, int ncol) const
+    int asked;            // 0 auto: the launched kernels choose by the colouring; else the form is given
+    int narrow;           // contacts a colour, on average, below which one CTA runs the sweeps ...
+    int narrow_contacts;  // ... of at most this many contacts
+    int wide;             // contacts a colour, on average, from which the grid runs
+    int many;             // from which the form's kernel with more groups a CTA runs (0: it has none)
+    __device__ __forceinline__ bool here(int kind, bool of_many, int nc, int ncol) const
     {
-        if (asked != 0) return true;
         const long long n = nc;
-        const bool narrow = nc <= kNarrowContacts && n < (long long)kNarrow * ncol;
-        return kind == (narrow ? kBlock : ncol > 0 && n >= (long long)wide * ncol ? kGrid : kCluster);
+        if (asked == 0) {
+            const bool one = nc <= narrow_contacts && n < (long long)narrow * ncol;
+            if (kind != (one ? kBlock : ncol > 0 && n >= (long long)wide * ncol ? kGrid : kCluster)) return false;
+        }
+        return of_many == (many > 0 && n >= (long long)many * ncol);
     }
 };
 
@@ -643,7 +646,7 @@ template <typename T, int kKind>
 __global__ void __launch_bounds__(sweep_threads<T, kKind>()) k_sweeps(SweepArgs<T> a)
 {
     const int ncol = a.stats[kNColors];
-    if (ncol == 0 || !a.form.here(kKind, a.nc, ncol)) return;  // uniform over the launch
+    if (ncol == 0 || !a.form.here(kKind, false, a.nc, ncol)) return;  // uniform over the launch
     __shared__ int s_start[kMaxColors], s_count[kMaxColors];
     const TaskTable tt = task_table(a, ncol, s_start, s_count);
     State<T> S{a.v, a.acc};
@@ -719,6 +722,115 @@ __global__ void __launch_bounds__(sweep_threads<T, kKind>()) k_sweeps(SweepArgs<
         for (int i = threadIdx.x; i < 6 * a.smem_bodies; i += blockDim.x) {
             a.acc[i] = S.acc[i];
             a.v[i] = S.v[i];
+        }
+}
+
+// The same update for a launch whose CTAs take several contacts each in every phase: there the time
+// is how many groups of a CTA are in flight, not one contact's chain, so everything is loaded where
+// it is used, which needs 64 registers a thread and lets a CTA have 64 groups (k_sweeps: 24 to 40,
+// float32 grid 64).  From kManyRounds rounds on, on average, this one runs: a launch of few CTAs that
+// was asked for, and the grid on scenes of 100 000 contacts.  Measured on a B200 (12 sweeps of 8
+// colours, us; k_sweeps / this one): one CTA, float64, 30 contacts a colour 267 / 298, 75 628 / 554,
+// 200 1 635 / 1 250, 1 250 10 497 / 7 058; a cluster of 8, 500 707 / 726, 1 250 1 629 / 1 312; a grid of
+// 16, 1 250 943 / 1 005, 2 500 1 529 / 1 359; a grid of 148, 25 000 2 047 / 1 524; float32, one CTA, 75
+// 457 / 468, 200 1 054 / 905, a cluster of 2, 200 679 / 734, 500 1 473 / 1 430.
+template <typename T>
+__device__ __forceinline__ T group_get(T x, int src, unsigned mask)
+{
+    return __shfl_sync(mask, x, src, kGroup);
+}
+
+template <typename T, int kKind>
+__device__ __forceinline__ void sweep_contact_many(const SweepArgs<T> &a, int c, int it, int l, unsigned mask)
+{
+    const int pa = a.pa[c], pb = a.pb[c];
+    const T lo[3] = {a.lam[3 * (size_t)c], a.lam[3 * (size_t)c + 1], a.lam[3 * (size_t)c + 2]};
+    // the six partial sums of u
+    T part = T(0), vs[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
+    if (l < 6) {
+        const int i = l % 3, side = l / 3, b = side == 0 ? pa : pb;
+        if (b >= 0) {
+            for (int j = 0; j < 6; ++j) vs[j] = shared_load<kKind>(a.v + 6 * (size_t)b + j);
+            const T *J = (side == 0 ? a.Ja : a.Jb) + 18 * (size_t)c + 6 * i;
+            T sacc = J[0] * vs[0];
+            for (int j = 1; j < 6; ++j) sacc = sacc + J[j] * vs[j];
+            part = sacc;
+        }
+    }
+    T u[3];
+    for (int i = 0; i < 3; ++i) {
+        const T sa = group_get(part, i, mask), sb = group_get(part, 3 + i, mask);
+        T ui = a.bias[3 * (size_t)c + i];
+        if (pa >= 0) ui = ui + sa;
+        if (pb >= 0) ui = ui + sb;
+        u[i] = ui;
+    }
+    T z[3], zn[3];
+    contact_z(u, lo, a.mu[c], a.rho[c], a.desaxce, a.soft, a.sep ? a.sep[c] : T(0), z);
+    proj(z, a.mu[c], zn);
+    if (a.trace) {
+        double *t = a.trace + kTraceWords * ((size_t)it * a.nc + c);
+        if (l == 0)
+            for (int k = 0; k < 3; ++k) {
+                t[k] = (double)lo[k];
+                t[18 + k] = (double)zn[k] - (double)lo[k];
+                t[33 + k] = (double)z[k];
+                t[36 + k] = (double)u[k];
+            }
+        if (l == 0 || l == 3)
+            for (int k = 0; k < 6; ++k) t[(l == 0 ? 3 : 9) + k] = (double)vs[k];
+    }
+    if (l < 3) a.lam[3 * (size_t)c + l] = l == 0 ? zn[0] : l == 1 ? zn[1] : zn[2];
+    if (l >= 12) return;
+    const int side = l / 6, k = l % 6, b = side == 0 ? pa : pb;
+    if (b < 0 || !a.dyn[b]) return;
+    const T *J = (side == 0 ? a.Ja : a.Jb) + 18 * (size_t)c;
+    const T *M = a.Minv + 36 * (size_t)b + 6 * k;
+    // row k of Minv (J^T l), minv_jt's order, for the new and the old impulse
+    T dn = T(0), dold = T(0);
+    for (int j = 0; j < 6; ++j) {
+        T tn = J[j] * zn[0];
+        tn = tn + J[6 + j] * zn[1];
+        tn = tn + J[12 + j] * zn[2];
+        T to = J[j] * lo[0];
+        to = to + J[6 + j] * lo[1];
+        to = to + J[12 + j] * lo[2];
+        if (j == 0) {
+            dn = M[0] * tn;
+            dold = M[0] * to;
+        } else {
+            dn = dn + M[j] * tn;
+            dold = dold + M[j] * to;
+        }
+    }
+    long long *p = a.acc + 6 * (size_t)b + k;
+    const long long sacc = shared_load<kKind>(p) + (quant(dn) - quant(dold));
+    shared_store<kKind>(p, sacc);
+    shared_store<kKind>(a.v + 6 * (size_t)b + k, a.vfree[6 * (size_t)b + k] + (T)unscale(sacc));
+}
+
+constexpr int kManyThreads = 1024;
+// rounds, in halves, from which k_sweeps_many runs (0: never)
+template <typename T, int kKind>
+constexpr int kManyRounds = sizeof(T) == 8 ? 5 : kKind == kGrid ? 0 : 9;
+
+template <typename T, int kKind>
+__global__ void __launch_bounds__(kManyThreads) k_sweeps_many(SweepArgs<T> a)
+{
+    const int ncol = a.stats[kNColors];
+    if (ncol == 0 || !a.form.here(kKind, true, a.nc, ncol)) return;  // uniform over the launch
+    const int nb = gridDim.x, groups = nb * (kManyThreads / kGroup);
+    const int g = ((int)threadIdx.x / kGroup) * nb + (int)blockIdx.x, l = (int)threadIdx.x % kGroup;
+    const unsigned mask = 0xFFFFu << (((int)threadIdx.x & 31) & ~(kGroup - 1));
+    unsigned int epoch = 0;
+    for (int it = 0; it < a.iters; ++it)
+        for (int ci = 0; ci < ncol; ++ci) {
+            const int s0 = a.cstart[ci], cnt = a.ccount[ci];
+            for (int t = g; t < cnt; t += groups) sweep_contact_many<T, kKind>(a, a.order[s0 + t], it, l, mask);
+            // in a cluster a warp's writes go out while others still compute: every warp's own release
+            if (kKind == kCluster) asm volatile("barrier.cluster.arrive.release;\n" ::: "memory");
+            else phase_arrive<kKind>(a, epoch);
+            if (!phase_wait<kKind>(a, epoch)) return;
         }
 }
 
@@ -1123,14 +1235,6 @@ int launch_kind(const void *fn, void **args, int kind, int ctas, int threads, si
     return check_launch(what);
 }
 
-template <typename A>
-int launch_phases(const void *fn, A &a, int kind, int ctas, int threads, size_t smem, const char *what, cudaStream_t s)
-{
-    if (kind == kGrid) cudaMemsetAsync(a.bar, 0, sizeof(uint32_t), s);  // the arrival count restarts every launch
-    void *args[] = {&a};
-    return launch_kind(fn, args, kind, ctas, threads, smem, what, s);
-}
-
 template <typename T>
 int color(const b2c_ncp_scene *sc, b2c_ncp_state *st, const b2c_ncp_params *p, cudaStream_t s)
 {
@@ -1155,12 +1259,18 @@ int color(const b2c_ncp_scene *sc, b2c_ncp_state *st, const b2c_ncp_params *p, c
     return launch_kind(fn, args, kind, ctas, kind == kGrid ? kColorGridThreads : kColorThreads, 0, "ncp_color", s);
 }
 
-// A phase kernel: its three forms (one CTA, a cluster, a cooperative grid), their threads, and the
-// most CTAs of the cluster and the grid that the device holds at once
+// A phase kernel: its three forms (one CTA, a cluster, a cooperative grid), their threads and shared
+// memory, the most CTAs of the cluster and the grid that the device holds at once, where the
+// automatic form changes (Form), and the kernels for many rounds of contacts a phase (NULL: none)
+// with the rounds, in halves, from which they run
 struct PhaseKernel {
     const void *fn[3];
     int threads[3];
+    size_t smem;
     int cluster_max, grid_max;
+    int narrow, narrow_contacts, wide;
+    const void *many[3];
+    int many_rounds[3];
 };
 
 // Runs a phase kernel in the form asked for (b2c_ncp_params.solve_blocks: 1 one CTA, n > 1 a
@@ -1170,16 +1280,23 @@ template <typename A>
 int run_phases(A &a, int asked, const PhaseKernel &k, size_t block_extra, const char *what, cudaStream_t s)
 {
     const int nc = a.nc;
-    a.form.asked = asked;
-    a.form.wide = k.cluster_max * (k.threads[kCluster] / kGroup);
+    a.form = Form{asked, k.narrow, k.narrow_contacts, k.wide, 0};
+    // a form's kernel and, where a colour can be wide enough, its kernel for many rounds: the
+    // colouring lets one of the two run (automatic: only the grid, the others change form before)
     auto launch = [&](int kind, int ctas) {
-        return launch_phases(k.fn[kind], a, kind, ctas, k.threads[kind],
-                             kTableBytes + (kind == kBlock ? block_extra : 0), what, s);
+        const bool has_many = k.many[kind] && (a.form.asked != 0 || kind == kGrid);
+        a.form.many = has_many ? std::max(1, ctas * (k.threads[kind] / kGroup) * k.many_rounds[kind] / 2) : 0;
+        void *args[] = {&a};
+        if (kind == kGrid) cudaMemsetAsync(a.bar, 0, sizeof(uint32_t), s);  // the arrival count restarts every launch
+        const int rc = launch_kind(k.fn[kind], args, kind, ctas, k.threads[kind],
+                                   k.smem + (kind == kBlock ? block_extra : 0), what, s);
+        if (rc != B2C_OK || !has_many || nc < a.form.many) return rc;
+        return launch_kind(k.many[kind], args, kind, ctas, kManyThreads, 0, what, s);
     };
     if (asked > 1 && std::min(asked, k.grid_max) > 1) return launch(kGrid, std::min(asked, k.grid_max));
     if (asked < 0 && std::min(-asked, k.cluster_max) >= 2) return launch(kCluster, std::min(-asked, k.cluster_max));
     if (asked != 0 || k.cluster_max < 2) {  // one CTA, asked for or all there is; without clusters the grid
-        const bool grid = asked == 0 && k.grid_max > 1 && nc > kNarrowContacts;
+        const bool grid = asked == 0 && k.grid_max > 1 && nc > k.narrow_contacts;
         a.form.asked = grid ? k.grid_max : 1;
         return grid ? launch(kGrid, k.grid_max) : launch(kBlock, 1);
     }
@@ -1187,8 +1304,8 @@ int run_phases(A &a, int asked, const PhaseKernel &k, size_t block_extra, const 
     // the device found lets one of them run (Form::here; the others return at once)
     if (k.grid_max < 2) a.form.wide = nc + 1;
     int rc = B2C_OK;
-    if (nc <= kNarrowContacts) rc = launch(kBlock, 1);
-    if (rc == B2C_OK && nc >= kNarrow) rc = launch(kCluster, k.cluster_max);
+    if (nc <= k.narrow_contacts) rc = launch(kBlock, 1);
+    if (rc == B2C_OK && nc >= k.narrow) rc = launch(kCluster, k.cluster_max);
     if (rc == B2C_OK && nc >= a.form.wide) rc = launch(kGrid, k.grid_max);
     return rc;
 }
@@ -1205,7 +1322,13 @@ int sweeps(const b2c_ncp_scene *sc, b2c_ncp_state *st, const b2c_ncp_params *p, 
     static const PhaseKernel k = {
         {(const void *)k_sweeps<T, kBlock>, (const void *)k_sweeps<T, kCluster>, (const void *)k_sweeps<T, kGrid>},
         {sweep_threads<T, kBlock>(), sweep_threads<T, kCluster>(), sweep_threads<T, kGrid>()},
-        cluster_size<T>(), grid_blocks<T>()};
+        kTableBytes,
+        std::min(cluster_size<T>(), cluster_size_of((const void *)k_sweeps_many<T, kCluster>, kManyThreads, 0)),
+        std::min(grid_blocks<T>(), grid_blocks_of((const void *)k_sweeps_many<T, kGrid>, kManyThreads, 0)),
+        16, 2048, cluster_size<T>() * (sweep_threads<T, kCluster>() / kGroup),
+        {(const void *)k_sweeps_many<T, kBlock>, (const void *)k_sweeps_many<T, kCluster>,
+         kManyRounds<T, kGrid> ? (const void *)k_sweeps_many<T, kGrid> : nullptr},
+        {kManyRounds<T, kBlock>, kManyRounds<T, kCluster>, kManyRounds<T, kGrid>}};
     return run_phases(a, p->solve_blocks, k, a.smem_bodies ? state : 0, "ncp_sweeps", s);
 }
 
@@ -1706,7 +1829,7 @@ template <int kKind>
 __global__ void __launch_bounds__(adj_threads<kKind>()) k_adj_sweeps(AdjArgs a)
 {
     const int ncol = a.stats[kNColors];
-    if (!a.form.here(kKind, a.nc, ncol)) return;  // uniform over the launch
+    if (!a.form.here(kKind, false, a.nc, ncol)) return;  // uniform over the launch
     const int nb = gridDim.x, nth = gridDim.x * blockDim.x;
     const int tid = ((((int)threadIdx.x >> 5) * nb + (int)blockIdx.x) << 5) | ((int)threadIdx.x & 31);
     const int gid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1850,11 +1973,12 @@ int adjoint_sweeps(const b2c_ncp_scene *sc, b2c_ncp_state *st, const b2c_ncp_par
     a.timeout_ns = p->barrier_timeout_ns > 0 ? p->barrier_timeout_ns : 1000000000LL;
     cudaMemsetAsync(vb, 0, sizeof(double) * 6 * (size_t)sc->n_b, s);
     if (trace) cudaMemsetAsync(st->res, 0, sizeof(double) * (size_t)sc->n_c, s);
+    static const int clusters = cluster_size_of((const void *)k_adj_sweeps<kCluster>, adj_threads<kCluster>(), kTableBytes);
     static const PhaseKernel k = {
         {(const void *)k_adj_sweeps<kBlock>, (const void *)k_adj_sweeps<kCluster>, (const void *)k_adj_sweeps<kGrid>},
-        {adj_threads<kBlock>(), adj_threads<kCluster>(), adj_threads<kGrid>()},
-        cluster_size_of((const void *)k_adj_sweeps<kCluster>, adj_threads<kCluster>(), kTableBytes),
-        grid_blocks_of((const void *)k_adj_sweeps<kGrid>, adj_threads<kGrid>(), kTableBytes)};
+        {adj_threads<kBlock>(), adj_threads<kCluster>(), adj_threads<kGrid>()}, kTableBytes, clusters,
+        grid_blocks_of((const void *)k_adj_sweeps<kGrid>, adj_threads<kGrid>(), kTableBytes),
+        16, 2048, clusters * (adj_threads<kCluster>() / kGroup), {}, {}};
     return run_phases(a, p->solve_blocks, k, 0, "ncp_adjoint", s);
 }
 
