@@ -1973,13 +1973,31 @@ int adjoint_sweeps(const b2c_ncp_scene *sc, b2c_ncp_state *st, const b2c_ncp_par
     a.timeout_ns = p->barrier_timeout_ns > 0 ? p->barrier_timeout_ns : 1000000000LL;
     cudaMemsetAsync(vb, 0, sizeof(double) * 6 * (size_t)sc->n_b, s);
     if (trace) cudaMemsetAsync(st->res, 0, sizeof(double) * (size_t)sc->n_c, s);
-    static const int clusters = cluster_size_of((const void *)k_adj_sweeps<kCluster>, adj_threads<kCluster>(), kTableBytes);
-    static const PhaseKernel k = {
-        {(const void *)k_adj_sweeps<kBlock>, (const void *)k_adj_sweeps<kCluster>, (const void *)k_adj_sweeps<kGrid>},
-        {adj_threads<kBlock>(), adj_threads<kCluster>(), adj_threads<kGrid>()}, kTableBytes, clusters,
-        grid_blocks_of((const void *)k_adj_sweeps<kGrid>, adj_threads<kGrid>(), kTableBytes),
-        16, 2048, clusters * (adj_threads<kCluster>() / kGroup), {}, {}};
-    return run_phases(a, p->solve_blocks, k, 0, "ncp_adjoint", s);
+    // the recorded sweeps (a group of lanes per contact, the task table in shared memory) and the
+    // sweeps at the final iterate (a thread per contact, the blocks through L1, from which a task table
+    // would take 96 KB: 80 contacts a colour in one CTA 781 us with it, 599 without).  A thread a
+    // contact makes one CTA the best form up to more contacts.  us for 20 reverse sweeps of 8 colours,
+    // one CTA / cluster / grid: 75 contacts a colour 982 / 1 113 / 1 362, 100 1 206 / 1 189 / 1 407, 125
+    // 1 343 / 1 178 / 1 436, 500 4 380 / 1 212 / 1 515, 1 000 - / 1 410 / 1 517, 1 250 - / 1 578 / 1 534.
+    auto phase_kernel = [](bool recorded) {
+        const size_t smem = recorded ? kTableBytes : 0;
+        const int clusters = cluster_size_of((const void *)k_adj_sweeps<kCluster>, adj_threads<kCluster>(), smem);
+        return PhaseKernel{
+            {(const void *)k_adj_sweeps<kBlock>, (const void *)k_adj_sweeps<kCluster>, (const void *)k_adj_sweeps<kGrid>},
+            {adj_threads<kBlock>(), adj_threads<kCluster>(), adj_threads<kGrid>()}, smem, clusters,
+            grid_blocks_of((const void *)k_adj_sweeps<kGrid>, adj_threads<kGrid>(), smem),
+            recorded ? 16 : 100, recorded ? 2048 : 16384,
+            recorded ? clusters * (adj_threads<kCluster>() / kGroup) : 1200, {}, {}};
+    };
+    static const PhaseKernel recorded = phase_kernel(true), implicit = phase_kernel(false);
+    PhaseKernel k = trace ? recorded : implicit;
+    int asked = p->solve_blocks;
+    if (!trace && asked < 0) {  // a cluster was asked for: that one, or one CTA below it
+        k.cluster_max = std::min(-asked, k.cluster_max);
+        k.grid_max = 1;
+        asked = 0;
+    }
+    return run_phases(a, asked, k, 0, "ncp_adjoint", s);
 }
 
 }  // namespace ncp
