@@ -267,8 +267,10 @@ enum Kind { kBlock = 0, kCluster = 1, kGrid = 2 };
 // contact's chain (~1.3 us) and how many contacts a group has to take one after the other, so the
 // form is the smallest launch that has a group for each contact of an average colour.  Measured
 // on a B200 (us per colour phase, float64; one CTA / cluster of 16 / grid of 148): 12 contacts a
-// colour 1.5 / 2.0 / 3.2, 22 2.4 / 2.0 / 3.2, 85 7.3 / 2.1 / 3.2, 300 24 / 2.3 / 3.3, 400 - / 4.3 / 3.4,
-// 5 000 - / 31 / 4.4.  In float32 the cluster has 640 groups and crosses at 500 to 600.
+// colour 1.5 / 2.0 / 3.2, 22 2.4 / 2.0 / 3.2, 85 7.3 / 2.1 / 3.2, 300 24 / 2.3 / 3.3, 350 - / 2.5 / 3.4,
+// 380 - / 3.6 / 3.4, 400 - / 4.6 / 3.4, 5 000 - / 31 / 4.4; float32 (640 groups in the cluster), 600 - /
+// 2.7 / 2.9, 635 - / 3.6 / 2.9, 700 - / 4.4 / 2.9.  The wider of the colours are over the average, so
+// the line is a thirty-second below the cluster's groups.
 struct Form {
     int asked;            // 0 auto: the launched kernels choose by the colouring; else the form is given
     int narrow;           // contacts a colour, on average, below which one CTA runs the sweeps ...
@@ -1325,7 +1327,7 @@ int sweeps(const b2c_ncp_scene *sc, b2c_ncp_state *st, const b2c_ncp_params *p, 
         kTableBytes,
         std::min(cluster_size<T>(), cluster_size_of((const void *)k_sweeps_many<T, kCluster>, kManyThreads, 0)),
         std::min(grid_blocks<T>(), grid_blocks_of((const void *)k_sweeps_many<T, kGrid>, kManyThreads, 0)),
-        16, 2048, cluster_size<T>() * (sweep_threads<T, kCluster>() / kGroup),
+        16, 2048, cluster_size<T>() * (sweep_threads<T, kCluster>() / kGroup) * 31 / 32,
         {(const void *)k_sweeps_many<T, kBlock>, (const void *)k_sweeps_many<T, kCluster>,
          kManyRounds<T, kGrid> ? (const void *)k_sweeps_many<T, kGrid> : nullptr},
         {kManyRounds<T, kBlock>, kManyRounds<T, kCluster>, kManyRounds<T, kGrid>}};
