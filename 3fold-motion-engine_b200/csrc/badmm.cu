@@ -36,8 +36,8 @@
 // Measured on a B200 (200 iterations of 8 CG steps and both gradients; before: a warp per problem,
 // the products matrix-free), B problems of 4 contacts and 18 coordinates: B = 64 5.8 -> 1.24 ms,
 // B = 4096 20.8 -> 1.31 ms (forward alone 11.7 -> 1.00), B = 16384 112 -> 3.1 ms; at B = 4096, 1
-// contact 10.2 -> 0.91 ms, 8 contacts 81.9 -> 5.3 ms.  Error against 64-bit arithmetic on the
-// batch of 4096: 1.2e-14 of the worst output's norm (before: 3.3e-13).
+// contact 10.2 -> 0.91 ms, 8 contacts 81.9 -> 5.3 ms.  Difference from a float64 restatement with
+// direct solves, on the batch of 4096: 1.2e-14 of the worst output's norm (before: 3.3e-13).
 #include <math_constants.h>
 
 #include "b2c_common.cuh"

@@ -1374,7 +1374,6 @@ struct AdjArgs {
     int nc, nb, iters, desaxce;
     const double *Ja, *Jb, *Minv, *mu, *rho, *lam, *u;
     double *trace;  // null: every reverse sweep at the final iterate (lam, u); else the recorded sweeps
-    const double *bias;
     const int *pa, *pb, *order, *cstart, *ccount, *dyn;
     double *gl, *vb, *vfree_b, *bias_b, *mu_b;
     double *Ja_b, *Jb_b, *Minv_b, *rho_b;  // the recorded form's adjoints of the blocks and step sizes
@@ -1954,7 +1953,6 @@ int adjoint_sweeps(const b2c_ncp_scene *sc, b2c_ncp_state *st, const b2c_ncp_par
     a.lam = (const double *)st->lam;
     a.u = (const double *)st->u;
     a.trace = trace;
-    a.bias = (const double *)sc->bias;
     a.Ja_b = Ja_b;
     a.Jb_b = Jb_b;
     a.Minv_b = Minv_b;

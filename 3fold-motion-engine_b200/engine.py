@@ -454,10 +454,12 @@ class RelaxedJacobiContactEngine(_BeadEngineBase):
         """One b2c_jacobi_solve on the current contacts between CUDA events (it moves the state on:
         call it last).  Returns (milliseconds, algorithmic bytes, counts).  Bytes per launch
         sequence, each array element read or written once per launch: a velocity iteration
-        (k_jacobi_velocity + k_jacobi_apply) moves 68 C + (76 + 16 x 12) E + 144 N, a position
+        (k_jacobi_velocity + k_jacobi_apply) moves 68 C + (76 + 16 x 6) E + 144 N, a position
         iteration 56 C + (76 + 16 x 6) E + 144 N -- C contacts, E their dynamic endpoints (a
-        body's xc, invM, invIw, v, w and its 6 int64 accumulators, 12 atomics per endpoint in the
-        velocity pass), N bodies (apply: 6 int64 read and cleared, v, w read and written)."""
+        body's xc, invM, invIw, v, w and its 6 int64 accumulators, an atomic each: a contact's
+        normal and friction deltas are added before it; a zero delta sends none, which this
+        count leaves out of account), N bodies (apply: 6 int64 read and cleared, v, w read and
+        written)."""
         h = self.header_dict()
         C = min(int(h["n_contacts"]), self.contact_capacity)
         bi = self.cbi[:C].long()
@@ -465,7 +467,7 @@ class RelaxedJacobiContactEngine(_BeadEngineBase):
         dyn = self.invM > 0
         E = int(dyn[bi].sum()) + int(((bj >= 0) & dyn[bj.clamp(min=0)]).sum())
         N = self.N
-        vel = 68 * C + (76 + 16 * 12) * E + 144 * N
+        vel = 68 * C + (76 + 16 * 6) * E + 144 * N
         pos = 56 * C + (76 + 16 * 6) * E + 144 * N
         s = torch.cuda.current_stream(self.dev)
         a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)

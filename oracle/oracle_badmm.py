@@ -3,7 +3,7 @@
 Only the tests and the bench's CPU-baseline leg may import this module.  It restates, in numpy
 float64 vectorised over the batch, the reference's ``BatchProxADMMGPU``
 (src/motion_engine/ncp/ncp_batch_gpu.py:918-1313, abbreviated NB below) so that the device
-solver (csrc/badmm.cu, one warp per problem) can be checked against it:
+solver (csrc/badmm.cu) can be checked against it:
 
 * set-up (NB:974-1000): b = J v_free, the int64 scale bound kappa, M^-1 J^T (k_mj NB:149-157),
   the dense Delassus G (k_gdense NB:160-167), its spectrum by cyclic Jacobi (k_jacobi
