@@ -299,7 +299,9 @@ typedef struct b2c_color_params {
                                 the device, the pairs of a colour; n > 0 = n CTAs
                                 with a grid barrier (1 = one CTA, block barriers); -n = a thread-block
                                 cluster of n CTAs with the hardware cluster barrier;
-                                B2C_SOLVE_SCENES = one CTA per scene (b2c_pairs' scene schedule) */
+                                B2C_SOLVE_SCENES = one CTA per scene (b2c_pairs' scene schedule).
+                                Engines that solve at the same time on several streams: -16 each,
+                                since 0 may take every SM */
     int64_t barrier_timeout_ns; /* grid-barrier wait limit */
     const float *body_mu;    /* (bodies) per-body friction, or NULL for the scalar mu: a body pair's
                                 contacts use sqrt(mu_a mu_b), a ground pair mu_a */
@@ -707,7 +709,7 @@ typedef struct b2c_admm_params {
     int32_t do_mu;          /* also the mu direction */
 } b2c_admm_params;
 
-/* dynamic shared memory of one warp's problems (-1 when nc or nv is out of range) */
+/* dynamic shared memory of a launch's CTA, one warp's problems (-1 when nc or nv is out of range) */
 B2C_API int64_t b2c_admm_smem_bytes(int32_t nc, int32_t nv);
 B2C_API int32_t b2c_admm_solve(const b2c_admm *a, const b2c_admm_params *p, b2c_stream s);
 
