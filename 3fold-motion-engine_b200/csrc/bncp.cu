@@ -31,11 +31,6 @@ namespace bncp {
 
 constexpr int kMaxN = 48;  // 3 x 16 contacts
 
-struct Env {
-    int n, nc;
-    const double *G, *b, *mu;
-};
-
 __device__ __forceinline__ double warp_sum(double v)
 {
 #pragma unroll

@@ -487,8 +487,10 @@ typedef struct b2c_ncp_state {
 typedef struct b2c_ncp_params {
     int32_t desaxce, soft, use_bias, color_cache;
     int32_t solve_blocks;      /* 0 auto (one CTA, a cluster or a grid of every co-resident CTA,
-                                  by the contacts of a colour; decided on the device), 1 one CTA, -n a cluster of n CTAs, n > 1 a
-                                  cooperative grid of n CTAs (at most the co-resident count) */
+                                  by the contacts of a colour; decided on the device), 1 one
+                                  CTA, -n a cluster of n CTAs (b2c_ncp_adjoint: one CTA where the
+                                  colours are narrow), n > 1 a cooperative grid of n CTAs (at
+                                  most the co-resident count) */
     int32_t pad;
     double softp[5];
     int64_t barrier_timeout_ns; /* grid-barrier wait limit (<= 0: 1 s) */
